@@ -1,6 +1,9 @@
 // C ABI: batched personalised PageRank (nwgpu_ppr_batched, include/nwgpu.h).
 // No counterpart in the reference; the single-vector personalised solve is
 // nwgpu_ppr_run in api.cu, and the looped baseline calls it k times.
+#include <cub/device/device_select.cuh>
+#include <thrust/iterator/counting_iterator.h>
+
 #include "handle.h"
 
 namespace nwgpu {
@@ -11,13 +14,37 @@ void PprBuffers::release(cudaStream_t s) {
   cg_exec = nullptr;
   cg = nullptr;
   void* ptrs[] = {tiling.tile_row, tiling.tile_nnz, rank, contrib[0], contrib[1], out, cpart, epart, res_part,
-                  spans, seeds, seeds_in, col_done, col_conv, col_iters, col_err, st, vbase, slot_map, slot_orig};
+                  end_bits, full_rows, tile_full, spans, seeds, seeds_in, col_done, col_conv, col_iters, col_err, st, vbase, slot_map, slot_orig};
   for (void* p : ptrs) pool_free(p, s);
   if (h_st) {
     cudaStreamSynchronize(s);  // no copy may still target the block when it is reused
     host_block_put(h_st);
   }
   *this = PprBuffers();
+}
+
+namespace {
+struct HasEntries {
+  const uint32_t* row_ptr;
+  __device__ bool operator()(uint32_t r) const { return row_ptr[r + 1] != row_ptr[r]; }
+};
+}  // namespace
+
+// rows = the graph's rows that have entries, ascending.
+static int list_full_rows(nwgpu_graph* g, uint32_t* rows) {
+  const thrust::counting_iterator<uint32_t> all(0u);
+  const HasEntries                          has{g->g.row_ptr};
+  unsigned int*                             num = nullptr;
+  void*                                     tmp = nullptr;
+  size_t                                    bytes = 0;
+  cudaError_t e = pool_alloc_n(&num, 1, g->stream);
+  if (e == cudaSuccess) e = cub::DeviceSelect::If(nullptr, bytes, all, rows, num, (int64_t)g->n, has, g->stream);
+  if (e == cudaSuccess) e = pool_alloc(&tmp, bytes, g->stream);
+  if (e == cudaSuccess) e = cub::DeviceSelect::If(tmp, bytes, all, rows, num, (int64_t)g->n, has, g->stream);
+  pool_free(tmp, g->stream);
+  pool_free(num, g->stream);
+  CK(e, "ppr rows");
+  return NWGPU_OK;
 }
 
 static int ensure_ppr(nwgpu_graph* g, int K) {
@@ -27,7 +54,6 @@ static int ensure_ppr(nwgpu_graph* g, int K) {
   const uint64_t n = g->n, nk = g->n * (uint64_t)K;
   CK(build_tiling(g->g.row_ptr, n, g->nnz, (uint32_t)kPprTileItems, &b.tiling, g->stream), "ppr tiling");
   const uint64_t T = b.tiling.num_tiles;
-  b.sweep_grid = ppr_sweep_grid(K, g->sms);
   b.finish_grid = g->sms * 4;
   CK(dalloc(g, &b.rank, nk), "cudaMalloc(ppr rank)");
   CK(dalloc(g, &b.contrib[0], nk), "cudaMalloc(ppr contrib)");
@@ -35,7 +61,7 @@ static int ensure_ppr(nwgpu_graph* g, int K) {
   CK(dalloc(g, &b.out, nk), "cudaMalloc(ppr out)");
   CK(dalloc(g, &b.cpart, (T + 1) * K), "cudaMalloc(ppr cpart)");
   CK(dalloc(g, &b.epart, (T + 1) * K), "cudaMalloc(ppr epart)");
-  CK(dalloc(g, &b.res_part, (uint64_t)(b.sweep_grid + b.finish_grid) * K), "cudaMalloc(ppr res)");
+  CK(dalloc(g, &b.res_part, (uint64_t)b.finish_grid * K), "cudaMalloc(ppr res)");
   CK(dalloc(g, &b.seeds, (uint64_t)K), "cudaMalloc(seeds)");
   CK(dalloc(g, &b.seeds_in, (uint64_t)K), "cudaMalloc(seeds)");
   CK(dalloc(g, &b.col_done, (uint64_t)K), "cudaMalloc(col flags)");
@@ -45,19 +71,31 @@ static int ensure_ppr(nwgpu_graph* g, int K) {
   CK(dalloc(g, &b.st, 1), "cudaMalloc(ppr state)");
   CK(dalloc(g, &b.slot_map, (uint64_t)K), "cudaMalloc(ppr slots)");
   CK(dalloc(g, &b.slot_orig, (uint64_t)K), "cudaMalloc(ppr slots)");
-  // rows crossing warp tiles, once per graph (counted in the state's ticket word, reset below)
+  // rows crossing tiles and the rows' last entries, once per graph
   CK(dalloc(g, &b.spans, T + 1), "cudaMalloc(ppr spans)");
+  CK(dalloc(g, &b.end_bits, g->nnz / 32 + 1), "cudaMalloc(ppr row ends)");
   {
-    unsigned int* cnt = &b.st->ticket;
-    CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned int), g->stream), "ppr spans");
-    CK(launch_ppr_spans(g->g.row_ptr, b.tiling.tile_row, b.tiling.tile_nnz, b.tiling.num_tiles, (uint32_t)kPprTileItems,
-                        b.spans, cnt, g->sms, g->stream),
-       "ppr spans");
-    unsigned int h_cnt = 0;
-    CK(cudaMemcpyAsync(&h_cnt, cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, g->stream), "ppr spans");
-    CK(cudaMemsetAsync(cnt, 0, sizeof(unsigned int), g->stream), "ppr spans");
-    CK(cudaStreamSynchronize(g->stream), "ppr spans");
-    b.num_spans = h_cnt;
+    unsigned int* cnt = nullptr;  // spans, rows that have entries
+    unsigned int  h_cnt[2] = {0, 0};
+    CK(dalloc(g, &cnt, 2), "cudaMalloc(ppr counts)");
+    cudaError_t e = launch_ppr_spans(g->g.row_ptr, b.tiling.tile_row, b.tiling.tile_nnz, b.tiling.num_tiles,
+                                     (uint32_t)kPprTileItems, b.spans, cnt, g->sms, g->stream);
+    if (e == cudaSuccess) e = launch_ppr_row_ends(g->g.row_ptr, n, b.end_bits, cnt + 1, g->sms, g->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(h_cnt, cnt, sizeof(h_cnt), cudaMemcpyDeviceToHost, g->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    pool_free(cnt, g->stream);
+    g->device_bytes -= (2 + kPad) * sizeof(unsigned int);
+    CK(e, "ppr spans");
+    b.num_spans = h_cnt[0];
+    b.num_full = h_cnt[1];
+  }
+  if (!g->relabelled && b.num_full < n) {  // input order: rows without entries anywhere
+    CK(dalloc(g, &b.full_rows, b.num_full), "cudaMalloc(ppr rows)");
+    CK(dalloc(g, &b.tile_full, T), "cudaMalloc(ppr rows)");
+    int rc = list_full_rows(g, b.full_rows);
+    if (rc) return rc;
+    CK(launch_ppr_tile_full(b.tiling.tile_row, (uint32_t)T, b.full_rows, b.num_full, b.tile_full, g->sms, g->stream),
+       "ppr rows");
   }
   static_assert(sizeof(PprState) <= kHostBlock, "state mirror fits a host block");
   CK(host_block_get((void**)&b.h_st), "cudaHostAlloc(ppr state)");
@@ -69,6 +107,11 @@ static int ensure_ppr(nwgpu_graph* g, int K) {
 int ppr_loop(nwgpu_graph* g, const PprArgs& a, int K, uint32_t k, float* ranks_nxk, float damping, uint64_t max_iters,
              const nwgpu_pr_options& opt, nwgpu_ppr_stats* stats, cudaStream_t s);
 
+static int padded_k(const nwgpu_graph* g, uint32_t k, int mode) {
+  const uint64_t items = g->n + g->nnz;
+  return ppr_padded_k(k, mode, ppr_few_tiles((items + kPprTileItems - 1) / kPprTileItems, g->sms));
+}
+
 static PprArgs make_ppr_args(nwgpu_graph* g, float damping) {
   PprBuffers& b = g->ppr;
   PprArgs     a = {};
@@ -78,6 +121,7 @@ static PprArgs make_ppr_args(nwgpu_graph* g, float damping) {
   a.tile_nnz = b.tiling.tile_nnz;
   a.num_tiles = b.tiling.num_tiles;
   a.tile_items = (uint32_t)kPprTileItems;
+  a.few_tiles = ppr_few_tiles(b.tiling.num_tiles, g->sms) ? 1u : 0u;
   a.deg = g->deg;
   a.rank = b.rank;
   a.contrib0 = b.contrib[0];
@@ -88,6 +132,10 @@ static PprArgs make_ppr_args(nwgpu_graph* g, float damping) {
   a.epi_grid = (uint32_t)b.finish_grid;
   a.n = g->n;
   a.K = (uint32_t)b.K;
+  a.end_bits = b.end_bits;
+  a.num_full = b.num_full;
+  a.full_rows = b.full_rows;
+  a.tile_full = b.tile_full;
   a.spans = b.spans;
   a.num_spans = b.num_spans;
 
@@ -126,7 +174,7 @@ extern "C" int nwgpu_ppr_batched(nwgpu_graph* g, const uint32_t* out_degree, con
   }
   for (uint32_t c = 0; c < k; ++c)
     if (h_seeds[c] >= g->n) return fail(NWGPU_ERR_INVALID_ARG, "seeds[%u] = %u >= n", c, h_seeds[c]);
-  const int      K = ppr_padded_k(k);
+  const int      K = padded_k(g, k, kPprSeeds);
   const uint64_t n = g->n;
   if (stats) {
     uint32_t* ci = stats->col_iterations;
@@ -166,9 +214,11 @@ namespace nwgpu {
 //
 // Narrowing (state narrow_at > 0): once at most narrow_at columns still run,
 // the device loop stops; every column's current ranks go to the output, the
-// running columns move into an n x K/2 layout (K' = 64 or 32), and the solve
-// goes on with the narrower kernels, launched from the host a few sweeps at a
-// time. The gather sums each column in the same order at every K, so the
+// running columns move into the narrowest layout that holds them (K' = 64, 32,
+// 16 or 8), and the solve goes on with the narrower kernels, launched from the
+// host a few sweeps at a time. Layouts of 32 columns or fewer are not narrowed
+// again: the move (two passes over the matrix and a host round trip) costs
+// about the sweeps it would save. The gather sums each column in the same order at every K, so the
 // result is the one the wide layout would give, at a fraction of the gather
 // traffic in the sweeps where most columns have stopped.
 int ppr_loop(nwgpu_graph* g, const PprArgs& a0, int K0, uint32_t k, float* ranks_nxk, float damping, uint64_t max_iters,
@@ -176,6 +226,7 @@ int ppr_loop(nwgpu_graph* g, const PprArgs& a0, int K0, uint32_t k, float* ranks
   PprBuffers&     b = g->ppr;
   const uint64_t  n = g->n;
   const int       mode = ppr_mode(a0);
+  const bool      few_tiles = a0.few_tiles != 0;
   const uint32_t* perm = g->relabelled ? g->g.perm : nullptr;
   float*          dst = opt.device_ptrs ? ranks_nxk : b.out;
   PprArgs         a = a0;
@@ -210,7 +261,7 @@ int ppr_loop(nwgpu_graph* g, const PprArgs& a0, int K0, uint32_t k, float* ranks
       if (b.cg) cudaGraphDestroy(b.cg);
       b.cg_exec = nullptr;
       CK(cudaGraphCreate(&b.cg, 0), "cudaGraphCreate");
-      CK(build_ppr_graph(b.cg, a, K, b.sweep_grid, b.st, &b.cg_exec), "ppr graph");
+      CK(build_ppr_graph(b.cg, a, K, ppr_sweep_grid(K, mode, few_tiles, g->sms), b.st, &b.cg_exec), "ppr graph");
       b.cg_damping = damping;
       b.cg_mode = mode;
     }
@@ -223,10 +274,11 @@ int ppr_loop(nwgpu_graph* g, const PprArgs& a0, int K0, uint32_t k, float* ranks
       if (b.h_st->done) break;
     }
   } else {
-    uint64_t launched = 0;
+    const int grid = ppr_sweep_grid(K, mode, few_tiles, g->sms);
+    uint64_t  launched = 0;
     for (;;) {
       const uint64_t batch = (max_iters - launched) < kGraphChunk ? (max_iters - launched) : kGraphChunk;
-      for (uint64_t i = 0; i < batch; ++i) CK(launch_ppr_sweep(a, K, b.sweep_grid, s), "ppr sweep");
+      for (uint64_t i = 0; i < batch; ++i) CK(launch_ppr_sweep(a, K, grid, s), "ppr sweep");
       launched += batch;
       CK(cudaMemcpyAsync(b.h_st, b.st, sizeof(PprState), cudaMemcpyDeviceToHost, s), "copy ppr state");
       CK(cudaStreamSynchronize(s), "ppr sweep loop");
@@ -243,7 +295,7 @@ int ppr_loop(nwgpu_graph* g, const PprArgs& a0, int K0, uint32_t k, float* ranks
     uint32_t nact = 0;
     for (int j = 0; j < K; ++j)
       if (!done[j]) map[nact++] = (uint32_t)j;
-    const int K2 = ppr_padded_k(nact ? nact : 1);
+    const int K2 = ppr_padded_k(nact ? nact : 1, mode, few_tiles);
     if (K2 >= K) return fail(NWGPU_ERR_CUDA, "narrowing found %u running columns of %d", nact, K);
     for (int j = 0; j < K2; ++j) orig2[j] = (uint32_t)j < nact ? orig[map[j]] : 0xffffffffu;
     CK(cudaMemcpyAsync(b.slot_map, map, nact * sizeof(uint32_t), cudaMemcpyHostToDevice, s), "copy slots");
@@ -277,7 +329,7 @@ int ppr_loop(nwgpu_graph* g, const PprArgs& a0, int K0, uint32_t k, float* ranks
     h.narrow_at = K > 32 ? (unsigned int)(K / 2) : 0u;
     *b.h_st = h;
     CK(cudaMemcpyAsync(b.st, b.h_st, sizeof(PprState), cudaMemcpyHostToDevice, s), "copy ppr state");
-    const int grid = ppr_sweep_grid(K, g->sms);
+    const int grid = ppr_sweep_grid(K, mode, few_tiles, g->sms);
     for (;;) {  // a few sweeps per check: the narrowed phases are short
       const uint64_t left = max_iters - b.h_st->iter, batch = left < 4 ? left : 4;
       for (uint64_t i = 0; i < batch; ++i) CK(launch_ppr_sweep(a, K, grid, s), "ppr sweep");
@@ -338,7 +390,7 @@ static int teleport_batched(nwgpu_graph* g, bool weighted, const uint32_t* out_d
   nwgpu_pr_options opt = {};
   if (options) memcpy(&opt, options, options->size && options->size < sizeof(opt) ? options->size : sizeof(opt));
   if (opt.launch > NWGPU_LAUNCH_STREAM) return fail(NWGPU_ERR_INVALID_ARG, "launch %u unknown", opt.launch);
-  const int      K = ppr_padded_k(k);
+  const int      K = padded_k(g, k, weighted ? kPprWeighted : kPprTeleports);
   const uint64_t n = g->n;
   if (stats) {
     uint32_t* ci = stats->col_iterations;

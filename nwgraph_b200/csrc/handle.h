@@ -69,15 +69,19 @@ struct WprBuffers {
 // Buffers of the batched personalised solve (K padded columns).
 struct PprBuffers {
   int             K = 0;
-  Tiling          tiling{};  // warp tiles of kPprTileItems
-  int             sweep_grid = 0, finish_grid = 0;
+  Tiling          tiling{};  // tiles of kPprTileItems
+  int             finish_grid = 0;  // epilogue CTAs
   float*          rank = nullptr;
   float*          contrib[2] = {nullptr, nullptr};
   float*          out = nullptr;  // n x K staging for the output
   float*          cpart = nullptr;
   float*          epart = nullptr;
   double*         res_part = nullptr;
-  uint4*          spans = nullptr;  // rows crossing warp tiles
+  uint32_t*       end_bits = nullptr;   // one bit per entry: the last of its row
+  uint32_t*       full_rows = nullptr;  // rows that have entries, where others lie between them
+  uint32_t*       tile_full = nullptr;  // per tile: its first row's place in full_rows
+  uint32_t        num_full = 0;
+  uint4*          spans = nullptr;  // rows crossing tiles
   uint32_t        num_spans = 0;
   uint32_t*       seeds = nullptr;
   uint32_t*       seeds_in = nullptr;

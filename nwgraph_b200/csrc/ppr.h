@@ -6,7 +6,8 @@
 
 namespace nwgpu {
 
-constexpr int kPprTileItems = 512;  // merge items per warp tile
+constexpr int kPprTileItems = 512;  // merge items per tile
+constexpr int kPprThreads = 256;    // gather CTA
 // What a batched solve's columns are: one-hot teleports at seeds; teleport
 // vectors on a weighted graph; teleport vectors on an unweighted graph.
 constexpr int kPprSeeds = 0, kPprWeighted = 1, kPprTeleports = 2;
@@ -27,10 +28,11 @@ struct PprState {
 struct PprArgs {
   const uint32_t* row_ptr;
   const uint32_t* col;
-  const uint32_t* tile_row;  // warp tiles of kPprTileItems
+  const uint32_t* tile_row;  // tiles of kPprTileItems
   const uint32_t* tile_nnz;
   uint32_t        num_tiles;
   uint32_t        tile_items;
+  uint32_t        few_tiles;  // ppr_few_tiles of the graph
   const uint32_t* deg;
   float*          rank;      // n x K
   float*          contrib0;  // n x K, ping-pong
@@ -41,7 +43,11 @@ struct PprArgs {
   uint32_t        epi_grid;
   uint64_t        n;
   uint32_t        K;          // padded column count
-  const uint4*    spans;      // rows crossing warp tiles: (row, first tile, last tile)
+  const uint32_t* end_bits;   // one bit per entry: the last of its row
+  uint32_t        num_full;   // rows that have entries
+  const uint32_t* full_rows;  // those rows, ascending; null where they are rows [0, num_full) (relabelled graphs)
+  const uint32_t* tile_full;  // with full_rows, per tile: the place in it of the first row >= tile_row[t]
+  const uint4*    spans;      // rows crossing tiles: (row, first tile, last tile)
   uint32_t        num_spans;
   const uint32_t* seeds;     // K internal seed ids (0xffffffff: padding column)
   uint32_t*       col_done;  // K flags
@@ -61,12 +67,21 @@ struct PprArgs {
   const float*                 vaux;
 };
 
-int         ppr_padded_k(uint32_t k);
+// Whether a graph of `tiles` tiles has at most one for each resident warp of the gather (a small graph).
+bool        ppr_few_tiles(uint64_t tiles, int sms);
+// Columns the solve's matrices get for a batch of k (0: k > 128); small graphs pad unweighted batches to 32.
+int         ppr_padded_k(uint32_t k, int mode, bool few_tiles);
 int         ppr_mode(const PprArgs& a);  // kPprSeeds, kPprWeighted or kPprTeleports
-// Rows crossing warp tiles (spans[count] = (row, first tile, last tile), any order).
+// Rows crossing tiles (spans[count] = (row, first tile, last tile), any order).
 cudaError_t launch_ppr_spans(const uint32_t* row_ptr, const uint32_t* tile_row, const uint32_t* tile_nnz, uint32_t T,
                              uint32_t D, uint4* spans, unsigned int* count, int sms, cudaStream_t s);
-int         ppr_sweep_grid(int K, int sms);
+// end_bits (zeroed, one bit per entry): the last entries of the rows; *full (zeroed) += rows that have entries.
+cudaError_t launch_ppr_row_ends(const uint32_t* row_ptr, uint64_t n, uint32_t* end_bits, unsigned int* full, int sms,
+                                cudaStream_t s);
+// tile_full[t] = place of the first row >= tile_row[t] in the ascending list rows[0, num).
+cudaError_t launch_ppr_tile_full(const uint32_t* tile_row, uint32_t T, const uint32_t* rows, uint32_t num,
+                                 uint32_t* tile_full, int sms, cudaStream_t s);
+int         ppr_sweep_grid(int K, int mode, bool few_tiles, int sms);  // gather CTAs
 cudaError_t launch_ppr_seeds(const uint32_t* seeds_in, uint32_t k, int K, const uint32_t* perm, const PprArgs& a,
                              cudaStream_t s);
 cudaError_t launch_ppr_init(const PprArgs& a, int K, uint64_t n, int sms, cudaStream_t s);

@@ -10,17 +10,202 @@
 // whose FP64 L1 change is below the threshold; its values are then frozen
 // while the other columns continue.
 //
-// One sweep is four kernels: the gather (merge-path tiles of W items per
-// warp, lanes owning K/32 columns each, rows of the contribution matrix
-// loaded U at a time with the next group in flight), the fix-up of rows that
-// cross tiles, a streaming epilogue over the n x K matrix (update, FP64
-// per-column residual, next contributions) and the per-column convergence
-// test.
+// One sweep is four kernels: the gather (merge-path tiles of W items, a group
+// of K/4 lanes per tile, so a warp walks 128/K tiles side by side), the fix-up
+// of rows that cross tiles, a streaming epilogue over the n x K matrix
+// (update, FP64 per-column residual, next contributions) and the per-column
+// convergence test. K is the batch size rounded up to 8, 16, 32, 64 or 128.
 #include "common.cuh"
 #include "engine.h"
 #include "ppr.h"
 
 namespace nwgpu {
+
+// ---------------------------------------------------------------------------
+// Gather. A tile is kPprTileItems merge items (entries and row ends); its
+// entries are summed in order into K running sums, and a finished row stores
+// its sums z into the output contribution matrix (the update, the residual and
+// the next contributions are the epilogue kernel's, so nothing in this loop
+// waits on a load other than the gathers). The first row of a tile that
+// started in an earlier tile leaves its partial in epart[t], the last row that
+// continues past the tile in cpart[t].
+//
+// A lane owns four columns (one 16-byte load per entry), so a tile takes
+// P = K/4 lanes and a warp walks 32/P tiles at once: the instructions per
+// entry fall with K, where a warp per tile would spend the same ~12 on an
+// entry whatever its width. Every column is summed in the same order at every
+// K: the tiles, the order within them and the crossing rows' partials do not
+// depend on it.
+//
+// Entries come in blocks of 16, aligned to 16 in the CSR: the group's first
+// lanes hold four column ids each (eight at K = 8, in 16-byte loads), and
+// weights likewise, passed on by shuffles. Which entries end a row is one bit
+// each (end_bits, built once per graph), so no row pointer is read per row.
+// The next block's ids load while this block's rows do, and the rows of one
+// sub-block of 8 entries are in flight while the sub-block before it is summed
+// (64 floats per lane, two CTAs of 256 threads per SM). Blocks that lie wholly
+// in their tiles, and sub-blocks in which no group's row ends, skip the
+// per-entry tests (a warp vote): the walk spends ~10 instructions on an entry
+// of each group instead of ~19, which made the gather 1.3x faster at K = 16.
+//
+// Bound by the bytes an SM takes from L2 (4 K per entry) and, below K = 32, by
+// instruction issue. Measured per sweep on RMAT scale 20 (31.4M entries),
+// against the warp-per-tile kernel below, which pads to 32 columns: K = 16 197
+// to 417 us, K = 32 301 to 419; weighted K = 16 215 to 829, K = 32 357 to 830
+// (that kernel loads every weight in every lane). Sub-blocks of 4 entries and
+// three CTAs per SM: 210 us at K = 16.
+// ---------------------------------------------------------------------------
+constexpr int kBlock = 16, kSub = 8;  // entries per block and sub-block
+
+// A lane holds N entries of the block: N = 16 / P for P < 4 lanes per group, else 4 (lanes sub < 4).
+template <int N>
+struct Block {
+  uint32_t id[N];  // column ids of entries base + N sub ..
+  float    w[N];   // their weights (weighted solves), 0 outside the tile
+  uint32_t mask;   // bits 0..15: entry base + u is in the tile; bits 16..31: it ends its row
+  bool     full;   // every group's block lies wholly in its tile (warp-uniform)
+};
+
+template <int N, bool WEIGHTED>
+__device__ __forceinline__ Block<N> load_block(const PprArgs& a, uint32_t base, uint32_t k0, uint32_t k1, int sub) {
+  Block<N>       b{};
+  const uint32_t lo = k0 > base ? k0 - base : 0u;  // entries [lo, hi) of the block are the tile's
+  const uint32_t hi = k1 > base ? min(k1 - base, (uint32_t)kBlock) : 0u;
+  b.full = __all_sync(kFullMask, lo == 0u && hi == (uint32_t)kBlock);
+  if (lo >= hi) return b;
+  const uint32_t in = ((1u << hi) - 1u) & ~((1u << lo) - 1u);
+  const uint32_t ends = __ldg(a.end_bits + (base >> 5)) >> (base & 31u);
+  b.mask = in | ((ends & in) << 16);
+#pragma unroll
+  for (int q = 0; q < N; q += 4) {
+    // the words reach at most 3 entries past the tile's last one: inside the arrays' padding
+    const uint32_t first = (uint32_t)(N * sub + q);
+    if (first >= hi || first + 4u <= lo) continue;
+    const uint4 id = ld_stream4(reinterpret_cast<const uint4*>(a.col + base + first));
+    b.id[q] = id.x;
+    b.id[q + 1] = id.y;
+    b.id[q + 2] = id.z;
+    b.id[q + 3] = id.w;
+    if (WEIGHTED) {
+      const float4 w = __ldcs(reinterpret_cast<const float4*>(a.w + base + first));
+      b.w[q] = (in >> first) & 1u ? w.x : 0.f;
+      b.w[q + 1] = (in >> first) & 2u ? w.y : 0.f;
+      b.w[q + 2] = (in >> first) & 4u ? w.z : 0.f;
+      b.w[q + 3] = (in >> first) & 8u ? w.w : 0.f;
+    }
+  }
+  return b;
+}
+
+// Rows of the block's entries kSub s .. kSub s + 7; entries outside the tile give 0.
+template <int K, int N>
+__device__ __forceinline__ void issue(float4 (&v)[kSub], const Block<N>& b, int s, int group,
+                                      const float* __restrict__ cin4, uint64_t pol) {
+  const uint32_t m = b.mask >> (kSub * s);
+  const float*   row[kSub];
+#pragma unroll
+  for (int u = 0; u < kSub; ++u)
+    row[u] = cin4 + (uint64_t)__shfl_sync(kFullMask, b.id[u % N], group * (K / 4) + (kSub * s + u) / N) * K;
+  if (b.full) {
+#pragma unroll
+    for (int u = 0; u < kSub; ++u) v[u] = ld_gather4(reinterpret_cast<const float4*>(row[u]), pol);
+  } else {
+#pragma unroll
+    for (int u = 0; u < kSub; ++u) {
+      v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (m & (1u << u)) v[u] = ld_gather4(reinterpret_cast<const float4*>(row[u]), pol);
+    }
+  }
+}
+
+template <int K, bool WEIGHTED>
+__global__ void __launch_bounds__(kPprThreads, 2) ppr_gather_kernel(const PprArgs a) {
+  constexpr int P = K / 4, G = 32 / P, N = P < 4 ? kBlock / P : 4;
+  static_assert(kBlock == 2 * kSub, "two sub-blocks in flight");
+  const int     lane = threadIdx.x & 31, sub = lane & (P - 1), group = lane / P;
+  PprState*     st = a.st;
+  if (a.use_cond && blockIdx.x == 0 && threadIdx.x == 0) cudaGraphSetConditional(a.cond, 0u);
+  if (*(volatile unsigned int*)&st->done) return;
+  const unsigned long long it = *(volatile unsigned long long*)&st->iter;
+  const float* __restrict__ cin4 = ((it & 1ull) ? a.contrib1 : a.contrib0) + 4 * sub;
+  float* __restrict__ cout4 = ((it & 1ull) ? a.contrib0 : a.contrib1) + 4 * sub;
+  const uint64_t pol = policy_evict_last();
+
+  const uint32_t gwarp = (blockIdx.x * kPprThreads + threadIdx.x) >> 5, nwarps = gridDim.x * (kPprThreads / 32);
+  // Fewer tiles than groups: spread them over all warps, for groups beside one another share their branches and
+  // their warp's issue slots (RMAT, K = 8: 40 and 48 us a sweep at scales 13 and 15, 55 at scale 14 with full warps).
+  const uint32_t per = (uint32_t)min((uint64_t)G, ((uint64_t)a.num_tiles + nwarps - 1u) / nwarps);
+  for (uint64_t t0 = (uint64_t)gwarp * per; t0 < a.num_tiles; t0 += (uint64_t)nwarps * per) {
+    const uint64_t t = (uint32_t)group < per ? t0 + (uint32_t)group : a.num_tiles;
+    uint32_t       r1 = 0u, k0 = 0u, k1 = 0u, row = 0u, pos = 0u;
+    bool           carry = false;
+    float*         dst = cout4;  // where the current row's sums go when it ends in this tile
+    if (t < a.num_tiles) {
+      row = a.tile_row[t];
+      r1 = a.tile_row[t + 1];
+      k0 = a.tile_nnz[t];
+      k1 = a.tile_nnz[t + 1];
+      const uint32_t s0 = __ldg(a.row_ptr + row), s1 = row < r1 ? __ldg(a.row_ptr + row + 1) : k1 + 1u;
+      carry = k1 > __ldg(a.row_ptr + r1);  // row r1 has entries here and ends in a later tile
+      bool cont = s0 < k0;                 // the first row started in an earlier tile
+      if (cont && s1 == k0) {              // and all its entries are there: only its end is this tile's
+        *reinterpret_cast<float4*>(a.epart + t * K + 4 * sub) = make_float4(0.f, 0.f, 0.f, 0.f);
+        cont = false;
+        ++row;
+      }
+      if (!WEIGHTED && a.full_rows) {  // rows without entries lie between the others: walk the list of those that have some
+        pos = a.tile_full[t] + (row > a.tile_row[t] ? 1u : 0u);
+        if (pos < a.num_full) row = a.full_rows[pos];
+      }
+      dst = cont ? a.epart + t * K + 4 * sub : cout4 + (uint64_t)row * K;
+    }
+    const uint32_t base0 = k0 & ~(uint32_t)(kBlock - 1);
+    const uint32_t blocks = __reduce_max_sync(kFullMask, k1 > k0 ? (k1 - base0 + kBlock - 1u) / kBlock : 0u);
+    float4         acc = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto           consume = [&](const float4(&v)[kSub], const Block<N>& blk, int s) {
+      const uint32_t ends = (blk.mask >> (16 + kSub * s)) & ((1u << kSub) - 1u);
+      float          w[kSub];
+#pragma unroll
+      for (int u = 0; u < kSub; ++u)
+        w[u] = WEIGHTED ? __shfl_sync(kFullMask, blk.w[u % N], group * P + (kSub * s + u) / N) : 1.f;
+      auto add = [&](int u) {
+        acc.x = WEIGHTED ? fmaf(w[u], v[u].x, acc.x) : acc.x + v[u].x;
+        acc.y = WEIGHTED ? fmaf(w[u], v[u].y, acc.y) : acc.y + v[u].y;
+        acc.z = WEIGHTED ? fmaf(w[u], v[u].z, acc.z) : acc.z + v[u].z;
+        acc.w = WEIGHTED ? fmaf(w[u], v[u].w, acc.w) : acc.w + v[u].w;
+      };
+      if (!__any_sync(kFullMask, ends != 0u)) {
+#pragma unroll
+        for (int u = 0; u < kSub; ++u) add(u);
+        return;
+      }
+#pragma unroll
+      for (int u = 0; u < kSub; ++u) {
+        add(u);
+        if (((ends >> u) & 1u) && row < r1) {
+          *reinterpret_cast<float4*>(dst) = acc;
+          acc = make_float4(0.f, 0.f, 0.f, 0.f);
+          if (!WEIGHTED && a.full_rows) row = ++pos < a.num_full ? a.full_rows[pos] : r1;
+          else ++row;
+          dst = cout4 + (uint64_t)row * K;
+        }
+      }
+    };
+    float4   va[kSub], vb[kSub];
+    Block<N> cur = load_block<N, WEIGHTED>(a, base0, k0, k1, sub);
+    issue<K>(va, cur, 0, group, cin4, pol);
+#pragma unroll 1
+    for (uint32_t b = 1; b <= blocks; ++b) {
+      const Block<N> nxt = load_block<N, WEIGHTED>(a, base0 + b * kBlock, k0, k1, sub);
+      issue<K>(vb, cur, 1, group, cin4, pol);
+      consume(va, cur, 0);
+      issue<K>(va, nxt, 0, group, cin4, pol);
+      consume(vb, cur, 1);
+      cur = nxt;
+    }
+    if (carry) *reinterpret_cast<float4*>(a.cpart + t * K + 4 * sub) = acc;
+  }
+}
 
 template <int K>
 struct Cols {
@@ -49,7 +234,16 @@ __device__ __forceinline__ void load_row(Cols<K>& out, const float* __restrict__
 }
 
 // ---------------------------------------------------------------------------
-// Gather: merge-path tiles of W items per warp. A warp walks its tile's
+// Gather, a warp per tile, lanes owning K/32 columns each: unweighted solves of
+// 64 and 128 columns and weighted ones of 128, where the walk above has one or
+// two tiles per warp and the loads, not the instructions, bound both (per
+// sweep on RMAT, against the walk above: scale 22, K = 64 2.28 to 2.33 ms; scale
+// 20, K = 128 0.97 to 1.02 ms; scale 17 weighted K = 128 154 to 160 us, but
+// scale 18 weighted K = 64 203 to 177); and unweighted solves of at most 32
+// columns on graphs with no more tiles than the walk above has warps
+// (ppr_few_tiles), where a tile's chain of loads is all of the time and a
+// warp has 16 rows of it in flight, not 8 (scale 15, 16 columns: 39 to 47 us;
+// scale 10: 35 to 36; scale 17, past the line: 67 to 61). A warp walks its tile's
 // entries in order, U rows of the contribution matrix per group, and loads
 // the next group while it sums the current one (2 * U * K * 4 bytes in flight
 // per warp: 4 KB for every K). Column ids and row ends of the tile are staged
@@ -80,7 +274,7 @@ __device__ __forceinline__ void load_weights(float (&wv)[U], const float* __rest
 }
 
 template <int K, int W, int U, bool WEIGHTED>
-__global__ void __launch_bounds__(256) ppr_gather_kernel(const PprArgs a) {
+__global__ void __launch_bounds__(256) ppr_gather_warp_kernel(const PprArgs a) {
   constexpr int P = Cols<K>::PER_LANE;
   constexpr int NWARP = 256 / 32;
   __shared__ uint32_t s_col[NWARP][W + 1];
@@ -163,8 +357,40 @@ __global__ void __launch_bounds__(256) ppr_gather_kernel(const PprArgs a) {
   }
 }
 
+// One bit per entry: it is the last of its row. full: rows that have entries.
+__global__ void ppr_row_ends_kernel(const uint32_t* __restrict__ row_ptr, uint64_t n, uint32_t* __restrict__ end_bits,
+                                    unsigned int* __restrict__ full) {
+  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  unsigned int   mine = 0;
+  for (uint64_t r = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; r < n; r += stride) {
+    const uint32_t e = row_ptr[r + 1];
+    if (e == row_ptr[r]) continue;
+    atomicOr(end_bits + ((e - 1u) >> 5), 1u << ((e - 1u) & 31u));
+    ++mine;
+  }
+  mine = __reduce_add_sync(kFullMask, mine);
+  if ((threadIdx.x & 31) == 0 && mine) atomicAdd(full, mine);
+}
+
+// Per tile: its first row's place in the list of rows that have entries.
+__global__ void ppr_tile_full_kernel(const uint32_t* __restrict__ tile_row, uint32_t T, const uint32_t* __restrict__ rows,
+                                     uint32_t num, uint32_t* __restrict__ tile_full) {
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < T; t += gridDim.x * blockDim.x) {
+    const uint32_t want = tile_row[t];
+    uint32_t       lo = 0, hi = num;
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (rows[mid] < want)
+        lo = mid + 1;
+      else
+        hi = mid;
+    }
+    tile_full[t] = lo;
+  }
+}
+
 // Rows that cross warp tiles are fixed by the tiling: listed once per graph
-// as (row, first tile, last tile). One warp per listed row sums its tile
+// as (row, first tile, last tile). K/4 lanes per listed row sum its tile
 // partials in tile order into z.
 __global__ void ppr_spans_kernel(const uint32_t* __restrict__ row_ptr, const uint32_t* __restrict__ tile_row,
                                  const uint32_t* __restrict__ tile_nnz, uint32_t T, uint32_t D, uint4* __restrict__ spans,
@@ -180,39 +406,40 @@ __global__ void ppr_spans_kernel(const uint32_t* __restrict__ row_ptr, const uin
 
 template <int K>
 __global__ void __launch_bounds__(256) ppr_fixup_kernel(const PprArgs a) {
-  constexpr int P = Cols<K>::PER_LANE;
+  constexpr int P = K / 4;  // lanes per row, four columns each
   PprState*     st = a.st;
   if (*(volatile unsigned int*)&st->done) return;
   const unsigned long long it = *(volatile unsigned long long*)&st->iter;
   float* __restrict__ cout = (it & 1ull) ? a.contrib0 : a.contrib1;
-  const int      lane = threadIdx.x & 31;
-  const uint32_t gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t sp = gwarp; sp < a.num_spans; sp += nwarps) {
-    const uint4 span = a.spans[sp];
+  const uint32_t th = blockIdx.x * blockDim.x + threadIdx.x, sub = th % P, ngroups = gridDim.x * blockDim.x / P;
+  for (uint32_t sp = th / P; sp < a.num_spans; sp += ngroups) {
+    const uint4   span = a.spans[sp];
+    const float4* part = reinterpret_cast<const float4*>(a.cpart) + sub;
     // 8 interleaved partial sums (tile u goes to sum (u - first) % 8), combined in order
-    float z[8][P];
+    float4 z[8];
 #pragma unroll
-    for (int j = 0; j < 8; ++j)
-#pragma unroll
-      for (int q = 0; q < P; ++q) z[j][q] = 0.f;
-    uint32_t u = span.y;
-    for (; u + 8 <= span.z; u += 8)
+    for (int j = 0; j < 8; ++j) z[j] = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t u = span.y; u < span.z; u += 8) {
 #pragma unroll
       for (int j = 0; j < 8; ++j)
-#pragma unroll
-        for (int q = 0; q < P; ++q) z[j][q] += __ldcg(a.cpart + (uint64_t)(u + j) * K + lane * P + q);
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-      if (u + j < span.z)
-#pragma unroll
-        for (int q = 0; q < P; ++q) z[j][q] += __ldcg(a.cpart + (uint64_t)(u + j) * K + lane * P + q);
-#pragma unroll
-    for (int q = 0; q < P; ++q) {
-      float t = 0.f;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) t += z[j][q];
-      cout[(uint64_t)span.x * K + lane * P + q] = t + __ldcg(a.epart + (uint64_t)span.z * K + lane * P + q);
+        if (u + j < span.z) {
+          const float4 x = __ldcg(part + (uint64_t)(u + j) * P);
+          z[j].x += x.x;
+          z[j].y += x.y;
+          z[j].z += x.z;
+          z[j].w += x.w;
+        }
     }
+    float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      t.x += z[j].x;
+      t.y += z[j].y;
+      t.z += z[j].z;
+      t.w += z[j].w;
+    }
+    const float4 e = __ldcg(reinterpret_cast<const float4*>(a.epart) + (uint64_t)span.z * P + sub);
+    reinterpret_cast<float4*>(cout)[(uint64_t)span.x * P + sub] = make_float4(t.x + e.x, t.y + e.y, t.z + e.z, t.w + e.w);
   }
 }
 
@@ -249,7 +476,9 @@ __global__ void __launch_bounds__(256) ppr_epilogue_kernel(const PprArgs a, uint
   if (any) {
     for (uint64_t x = x0; x < total; x += stride) {
       const uint32_t i = (uint32_t)(x / C4);
-      const float4   z = __ldcs(reinterpret_cast<const float4*>(cout) + x);
+      // the gather leaves the rows without entries alone: their sum is 0
+      const bool     full = a.full_rows ? __ldg(a.row_ptr + i) != __ldg(a.row_ptr + i + 1) : i < a.num_full;
+      const float4   z = full ? __ldcs(reinterpret_cast<const float4*>(cout) + x) : make_float4(0.f, 0.f, 0.f, 0.f);
       const float4   old = __ldcs(reinterpret_cast<const float4*>(a.rank) + x);
       // weighted: divide by the out-weight sum; the base terms are (1 - d) t
       const float    dg = EPI == kPprWeighted ? __ldg(a.vaux + i) : (float)__ldg(a.deg + i);
@@ -452,6 +681,18 @@ cudaError_t launch_ppr_spans(const uint32_t* row_ptr, const uint32_t* tile_row, 
   return cudaGetLastError();
 }
 
+cudaError_t launch_ppr_row_ends(const uint32_t* row_ptr, uint64_t n, uint32_t* end_bits, unsigned int* full, int sms,
+                                cudaStream_t s) {
+  ppr_row_ends_kernel<<<sms * 8, 256, 0, s>>>(row_ptr, n, end_bits, full);
+  return cudaGetLastError();
+}
+
+cudaError_t launch_ppr_tile_full(const uint32_t* tile_row, uint32_t T, const uint32_t* rows, uint32_t num,
+                                 uint32_t* tile_full, int sms, cudaStream_t s) {
+  ppr_tile_full_kernel<<<sms * 4, 256, 0, s>>>(tile_row, T, rows, num, tile_full);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_ppr_seeds(const uint32_t* seeds_in, uint32_t k, int K, const uint32_t* perm, const PprArgs& a,
                              cudaStream_t s) {
   ppr_seed_kernel<<<1, 128, 0, s>>>(seeds_in, k, K, perm, a);
@@ -479,12 +720,19 @@ cudaError_t launch_ppr_output_slots(const float* rank, const uint32_t* perm, uin
 
 __global__ void ppr_arm_kernel(PprState* st) { st->chunk_end = st->iter + kGraphChunk; }
 
-// Rows per group: U * K = 512 floats, 2 KB of rows per group (16 floats per lane).
 template <int K, int EPI>
 struct PprKernels {
-  static constexpr int U = 512 / K;
-  static void*         fn(int which) {
-    return which == 0   ? (void*)ppr_gather_kernel<K, kPprTileItems, U, EPI == kPprWeighted>
+  static constexpr bool kW = EPI == kPprWeighted;
+  // Rows per group: U * K = 512 floats, 2 KB of rows per group (16 floats per lane).
+  static void* gather(bool few_tiles) {
+    if constexpr (K > (kW ? 64 : 32)) return (void*)ppr_gather_warp_kernel<K, kPprTileItems, 512 / K, kW>;
+    if constexpr (K == 32 && !kW)
+      if (few_tiles) return (void*)ppr_gather_warp_kernel<K, kPprTileItems, 512 / K, kW>;
+    if constexpr (K <= (kW ? 64 : 32)) return (void*)ppr_gather_kernel<K, kW>;
+    return nullptr;
+  }
+  static void* fn(int which, bool few_tiles) {
+    return which == 0   ? gather(few_tiles)
            : which == 1 ? (void*)ppr_fixup_kernel<K>
            : which == 2 ? (void*)ppr_epilogue_kernel<K, EPI>
                         : (void*)ppr_finish_kernel<K>;
@@ -492,44 +740,55 @@ struct PprKernels {
 };
 
 template <int K>
-static void* ppr_fn_k(int which, int mode) {
-  return mode == kPprWeighted    ? PprKernels<K, kPprWeighted>::fn(which)
-         : mode == kPprTeleports ? PprKernels<K, kPprTeleports>::fn(which)
-                                 : PprKernels<K, kPprSeeds>::fn(which);
+static void* ppr_fn_k(int which, int mode, bool few_tiles) {
+  return mode == kPprWeighted    ? PprKernels<K, kPprWeighted>::fn(which, few_tiles)
+         : mode == kPprTeleports ? PprKernels<K, kPprTeleports>::fn(which, few_tiles)
+                                 : PprKernels<K, kPprSeeds>::fn(which, few_tiles);
 }
 
 // kernel 0 gather, 1 fix-up, 2 epilogue, 3 finish, for the solve's mode
-static void* ppr_fn(int K, int which, int mode = kPprSeeds) {
+static void* ppr_fn(int K, int which, int mode, bool few_tiles) {
   switch (K) {
-    case 32: return ppr_fn_k<32>(which, mode);
-    case 64: return ppr_fn_k<64>(which, mode);
-    case 128: return ppr_fn_k<128>(which, mode);
+    case 8: return ppr_fn_k<8>(which, mode, few_tiles);
+    case 16: return ppr_fn_k<16>(which, mode, few_tiles);
+    case 32: return ppr_fn_k<32>(which, mode, few_tiles);
+    case 64: return ppr_fn_k<64>(which, mode, few_tiles);
+    case 128: return ppr_fn_k<128>(which, mode, few_tiles);
     default: return nullptr;
   }
 }
 
 int ppr_mode(const PprArgs& a) { return a.w ? kPprWeighted : (a.vbase ? kPprTeleports : kPprSeeds); }
 
-// Grid of each kernel: gather persistent at its occupancy, fix-up one warp
+// Grid of each kernel: gather persistent at its occupancy, fix-up K/4 lanes
 // per row crossing tiles, epilogue epi_grid CTAs, finish one warp per column.
 static int K_of(const PprArgs& a) { return (int)a.K; }
 static dim3 ppr_grid(const PprArgs& a, int which, int sweep_grid) {
   if (which == 0) return dim3((unsigned)sweep_grid);
-  if (which == 1) return dim3(a.num_spans ? (a.num_spans + 7u) / 8u : 1u);
+  if (which == 1) return dim3(a.num_spans ? (unsigned)(((uint64_t)a.num_spans * (a.K / 4u) + 255u) / 256u) : 1u);
   if (which == 2) return dim3(a.epi_grid);
   return dim3((unsigned)(K_of(a) / 8));
 }
 
-int ppr_padded_k(uint32_t k) { return k <= 32 ? 32 : (k <= 64 ? 64 : (k <= 128 ? 128 : 0)); }
+bool ppr_few_tiles(uint64_t tiles, int sms) { return tiles <= (uint64_t)sms * (2 * kPprThreads / 32); }
 
-int ppr_sweep_grid(int K, int sms) {
+int ppr_padded_k(uint32_t k, int mode, bool few_tiles) {
+  if (few_tiles && mode != kPprWeighted && k <= 32) return 32;
+  return k <= 8 ? 8 : k <= 16 ? 16 : k <= 32 ? 32 : k <= 64 ? 64 : k <= 128 ? 128 : 0;
+}
+
+int ppr_sweep_grid(int K, int mode, bool few_tiles, int sms) {
   int nb = 0;
-  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ppr_fn(K, 0), 256, 0) != cudaSuccess || nb < 1) nb = 1;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, ppr_fn(K, 0, mode, few_tiles), kPprThreads, 0) != cudaSuccess ||
+      nb < 1)
+    nb = 1;
   return sms * nb;
 }
 
 cudaError_t launch_ppr_init(const PprArgs& a, int K, uint64_t n, int sms, cudaStream_t s) {
   switch (K) {
+    case 8: ppr_init_kernel<8><<<sms * 8, 256, 0, s>>>(a, n); break;
+    case 16: ppr_init_kernel<16><<<sms * 8, 256, 0, s>>>(a, n); break;
     case 32: ppr_init_kernel<32><<<sms * 8, 256, 0, s>>>(a, n); break;
     case 64: ppr_init_kernel<64><<<sms * 8, 256, 0, s>>>(a, n); break;
     case 128: ppr_init_kernel<128><<<sms * 8, 256, 0, s>>>(a, n); break;
@@ -541,6 +800,8 @@ cudaError_t launch_ppr_init(const PprArgs& a, int K, uint64_t n, int sms, cudaSt
 cudaError_t launch_ppr_winit(const PprArgs& a, int K, const float* t_in, uint32_t k, const uint32_t* inv, uint64_t n,
                              float* vbase, int sms, cudaStream_t s) {
   switch (K) {
+    case 8: ppr_winit_kernel<8><<<sms * 8, 256, 0, s>>>(a, t_in, k, inv, n, vbase); break;
+    case 16: ppr_winit_kernel<16><<<sms * 8, 256, 0, s>>>(a, t_in, k, inv, n, vbase); break;
     case 32: ppr_winit_kernel<32><<<sms * 8, 256, 0, s>>>(a, t_in, k, inv, n, vbase); break;
     case 64: ppr_winit_kernel<64><<<sms * 8, 256, 0, s>>>(a, t_in, k, inv, n, vbase); break;
     case 128: ppr_winit_kernel<128><<<sms * 8, 256, 0, s>>>(a, t_in, k, inv, n, vbase); break;
@@ -552,6 +813,8 @@ cudaError_t launch_ppr_winit(const PprArgs& a, int K, const float* t_in, uint32_
 cudaError_t launch_ppr_output(const float* rank, const uint32_t* perm, uint64_t n, int K, uint32_t k, float* out,
                               int sms, cudaStream_t s) {
   switch (K) {
+    case 8: ppr_output_kernel<8><<<sms * 8, 256, 0, s>>>(rank, perm, n, k, out); break;
+    case 16: ppr_output_kernel<16><<<sms * 8, 256, 0, s>>>(rank, perm, n, k, out); break;
     case 32: ppr_output_kernel<32><<<sms * 8, 256, 0, s>>>(rank, perm, n, k, out); break;
     case 64: ppr_output_kernel<64><<<sms * 8, 256, 0, s>>>(rank, perm, n, k, out); break;
     case 128: ppr_output_kernel<128><<<sms * 8, 256, 0, s>>>(rank, perm, n, k, out); break;
@@ -565,7 +828,7 @@ cudaError_t launch_ppr_sweep(const PprArgs& a, int K, int sweep_grid, cudaStream
   for (int w = 0; w < 4; ++w) {
     uint64_t    n = a.n;
     void*       eargs[] = {(void*)&a, (void*)&n};
-    cudaError_t e = cudaLaunchKernel(ppr_fn(K, w, ppr_mode(a)), ppr_grid(a, w, sweep_grid), dim3(256),
+    cudaError_t e = cudaLaunchKernel(ppr_fn(K, w, ppr_mode(a), a.few_tiles != 0), ppr_grid(a, w, sweep_grid), dim3(256),
                                      w == 2 ? eargs : args, 0, s);
     if (e != cudaSuccess) return e;
   }
@@ -602,7 +865,7 @@ cudaError_t build_ppr_graph(cudaGraph_t g, const PprArgs& proto, int K, int swee
   cudaGraphNode_t      prev = nullptr;
   for (int w = 0; w < 4; ++w) {
     cudaKernelNodeParams kp2 = {};
-    kp2.func = ppr_fn(K, w, ppr_mode(a));
+    kp2.func = ppr_fn(K, w, ppr_mode(a), a.few_tiles != 0);
     kp2.gridDim = ppr_grid(a, w, sweep_grid);
     kp2.blockDim = dim3(256);
     kp2.kernelParams = w == 2 ? eargs : args;
