@@ -189,6 +189,7 @@ int check_device(int* dev_out, int* sms_out) {
     g_config_err = configure_sweep_kernels();
     if (g_config_err == cudaSuccess) g_config_err = configure_binned_kernels();
     if (g_config_err == cudaSuccess) g_config_err = configure_blocked_kernels();
+    if (g_config_err == cudaSuccess) g_config_err = configure_resident_kernel();
   });
   if (g_config_err != cudaSuccess) return cuda_fail(g_config_err, "configure kernels");
   *dev_out = dev;
@@ -222,6 +223,7 @@ int ensure_solve_buffers(nwgpu_graph* g) {
   CK(dalloc(g, &g->err_hist, g->err_cap), "cudaMalloc(err_hist)");
   static_assert(sizeof(PrState) <= kHostBlock, "state mirror fits a host block");
   CK(host_block_get((void**)&g->h_st), "cudaHostAlloc(state)");
+  CK(cudaHostGetDevicePointer((void**)&g->d_hst, g->h_st, 0), "cudaHostGetDevicePointer(state)");
   CK(host_block_get((void**)&g->h_abort), "cudaHostAlloc(abort)");
   CK(cudaHostGetDevicePointer((void**)&g->d_abort, g->h_abort, 0), "cudaHostGetDevicePointer(abort)");
   CK(cudaEventCreate(&g->ev0), "cudaEventCreate");
@@ -377,6 +379,63 @@ void BinPlan::release(cudaStream_t s) {
   *this = BinPlan();
 }
 
+void ResidentPlan::release(cudaStream_t s) {
+  pool_free(bounds, s);
+  pool_free(sync, s);
+  pool_free(part, s);
+  *this = ResidentPlan();
+}
+
+// The resident solve's plan, once per graph: relabelled graphs on the binned
+// sweep (not one that NWGPU_SWEEP names) of which every CTA's rows and entries
+// fit its shared memory. The hubs staged beside them are those that save the
+// most: a sweep's gathers past them cost about a clock each per SM, staging
+// sixteen of them one (both from the L2 paths' rates), and the share of
+// gathers that hit the first H ids is the share of entries in their rows
+// (exact where the graph is symmetric).
+static int ensure_resident(nwgpu_graph* g) {
+  ResidentPlan& p = g->resident;
+  if (p.tried) return NWGPU_OK;
+  p.tried = true;
+  if (!g->relabelled || !g->plan.ok || g->bplan.ok || g->n == 0 || g->nnz > kResidentMaxEntries ||
+      g->n > kResidentMaxEntries || getenv("NWGPU_SWEEP"))
+    return NWGPU_OK;
+  const int      C = resident_ctas(g->n, g->nnz, g->sms);
+  const uint64_t words = 2 * ((uint64_t)C + 1) + kNumResidentHubs;
+  CK(dalloc(g, &p.bounds, (uint64_t)C + 1), "cudaMalloc(resident bounds)");
+  CK(dalloc(g, &p.sync, 2), "cudaMalloc(resident counters)");
+  CK(dalloc(g, &p.part, 2 * ((uint64_t)C + 1)), "cudaMalloc(resident partials)");
+  std::vector<uint32_t> h(words);
+  uint32_t*             d = nullptr;
+  cudaError_t           e = pool_alloc_n(&d, words, g->stream);
+  if (e == cudaSuccess) e = launch_resident_bounds(g->g.row_ptr, g->n, g->nnz, C, p.bounds, d, g->stream);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), d, words * sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+  pool_free(d, g->stream);
+  CK(e, "resident bounds");
+  uint64_t most = 0, most_entries = 0;
+  for (int c = 0; c < C; ++c) {
+    const uint64_t E = h[C + 2 + c] - h[C + 1 + c], R = h[c + 1] - h[c];
+    most = std::max(most, resident_words(E, R));
+    most_entries = std::max(most_entries, E);
+  }
+  const uint64_t limit = resident_smem_limit() / 4u;
+  if (most > limit) return NWGPU_OK;
+  double best = (double)most_entries;
+  for (uint32_t i = 0; i < kNumResidentHubs; ++i) {
+    const uint64_t H = std::min<uint64_t>(kResidentHubStep * (i + 1u), g->n) & ~3ull;
+    const double   cost = H / 16.0 + most_entries * (1.0 - (double)h[2 * (C + 1) + i] / (double)(g->nnz ? g->nnz : 1));
+    if (cost < best && most + H <= limit) {
+      best = cost;
+      p.hub_ids = (uint32_t)H;
+    }
+  }
+  p.smem_bytes = (uint32_t)(most + p.hub_ids) * 4u;
+  p.ctas = C;
+  p.ok = true;
+  return NWGPU_OK;
+}
+
 // Sweep grid of a binned solve: the plan's, except the weighted and adjoint
 // sweeps, which always run in the hot launch shape.
 int binned_grid(nwgpu_graph* g, const BinPlan& p, int mode) {
@@ -526,6 +585,95 @@ nwgpu_pr_options read_options(const nwgpu_pr_options* options) {
   return opt;
 }
 
+// The caller's statistics of a finished solve (ev0 to ev1), and its status.
+static int report_solve(nwgpu_graph* g, const PrState& fin, nwgpu_pr_stats* stats, cudaStream_t s) {
+  if (stats) {
+    float ms = 0.f;
+    cudaEventElapsedTime(&ms, g->ev0, g->ev1);
+    stats->iterations = fin.iter;
+    stats->final_error = fin.last_error;
+    stats->converged = (int32_t)fin.converged;
+    stats->device_ms = ms;
+    stats->ms_per_iter = fin.iter ? ms / (double)fin.iter : 0.0;
+    stats->gteps = ms > 0 ? (double)g->nnz * (double)fin.iter / (ms * 1e6) : 0.0;
+    if (stats->errors && stats->errors_cap) {
+      uint64_t m = fin.iter < stats->errors_cap ? fin.iter : stats->errors_cap;
+      if (m > g->err_cap) m = g->err_cap;
+      if (m) {
+        CK(cudaMemcpyAsync(stats->errors, g->err_hist, m * sizeof(double), cudaMemcpyDeviceToHost, s), "copy errors");
+        CK(cudaStreamSynchronize(s), "copy errors");
+      }
+    }
+  }
+  if (fin.aborted) return fail(NWGPU_ERR_ABORTED, "solve aborted after %llu sweeps", (unsigned long long)fin.iter);
+  return NWGPU_OK;
+}
+
+// A plain or single-seed solve as resident launches (one, unless it takes more
+// than kGraphChunk sweeps). *ran stays false, with nothing done, where the
+// device cannot hold the grid at once; the caller then runs the sweep loop.
+static int solve_resident(nwgpu_graph* g, const uint32_t* out_degree, float* ranks, float damping, float threshold,
+                          uint64_t max_iters, bool device_ptrs, int teleport, uint32_t seed, float init, float base,
+                          cudaStream_t s, nwgpu_pr_stats* stats, bool* ran) {
+  ResidentPlan&     p = g->resident;
+  const BinnedArgs& b = g->plan.bin;
+  const uint64_t    n = g->n;
+  ResidentArgs      a = {};
+  a.row_ptr = g->g.row_ptr;
+  a.col = g->g.col;
+  a.inv = g->g.inv;
+  a.deg = device_ptrs ? out_degree : g->stage_u32;
+  a.out = device_ptrs ? ranks : reinterpret_cast<float*>(g->stage_u32);  // the degrees are read before any rank is out
+  a.rank = g->rank;
+  a.contrib0 = g->contrib[0];
+  a.contrib1 = g->contrib[1];
+  a.bounds = p.bounds;
+  a.sync = p.sync;
+  a.part = p.part;
+  a.state = g->d_hst;
+  a.err_hist = g->err_hist;
+  a.err_cap = g->err_cap;
+  a.abort_word = g->d_abort;
+  a.max_iters = max_iters;
+  a.threshold = (double)threshold;
+  a.damping = damping;
+  a.base = base;
+  a.init = init;
+  a.teleport = teleport;
+  a.seed = seed;
+  a.long_row = b.long_row;
+  a.chunk = b.chunk;
+  a.bin0_rows = b.bin0_rows;
+  a.num_long_rows = b.num_long_rows;
+  memcpy(a.bin_row_begin, b.bin_row_begin, sizeof(a.bin_row_begin));
+  memcpy(a.bin_row_end, b.bin_row_end, sizeof(a.bin_row_end));
+  a.hub_ids = p.hub_ids;
+  if (!device_ptrs)
+    CK(cudaMemcpyAsync(g->stage_u32, out_degree, n * sizeof(uint32_t), cudaMemcpyHostToDevice, s), "copy out_degree");
+  *g->h_st = PrState{};
+  CK(cudaEventRecord(g->ev0, s), "cudaEventRecord");
+  do {
+    a.turn = p.turn;
+    a.chunk_end = a.iter0 + kGraphChunk;
+    const cudaError_t e = launch_resident(a, p.ctas, p.smem_bytes, s);
+    if (a.iter0 == 0 && (e == cudaErrorCooperativeLaunchTooLarge || e == cudaErrorNotSupported)) {
+      cudaGetLastError();
+      p.ok = false;
+      return NWGPU_OK;
+    }
+    CK(e, "pr_resident");
+    *ran = true;
+    p.turn ^= 1u;
+    CK(cudaEventRecord(g->ev1, s), "cudaEventRecord");
+    if (!device_ptrs) CK(cudaMemcpyAsync(ranks, a.out, n * sizeof(float), cudaMemcpyDeviceToHost, s), "copy ranks");
+    CK(cudaStreamSynchronize(s), "pr_resident");
+    a.iter0 = g->h_st->iter;
+  } while (!g->h_st->done);
+  const PrState fin = *g->h_st;
+  if (fin.fault) return fail(NWGPU_ERR_CUDA, "a bounded device wait gave up (fault word %u)", fin.fault);
+  return report_solve(g, fin, stats, s);
+}
+
 // Shared body of nwgpu_pr_run (uniform teleport) and nwgpu_ppr_run (one-hot).
 int solve_single(nwgpu_graph* g, const uint32_t* out_degree, float* ranks, float damping, float threshold,
                  uint64_t max_iters, const nwgpu_pr_options* options, nwgpu_pr_stats* stats, int teleport,
@@ -567,6 +715,15 @@ int solve_single(nwgpu_graph* g, const uint32_t* out_degree, float* ranks, float
   if (rc) return rc;
   *(volatile unsigned int*)g->h_abort = 0u;
   trace.mark("solve buffers");
+  if (opt.launch == NWGPU_LAUNCH_GRAPH) {
+    if ((rc = ensure_resident(g))) return rc;
+    if (g->resident.ok) {
+      bool ran = false;
+      rc = solve_resident(g, out_degree, ranks, damping, threshold, max_iters, opt.device_ptrs != 0, teleport, seed_in, init,
+                          base, s, stats, &ran);
+      if (rc || ran) return rc;
+    }
+  }
   if ((rc = load_degrees(g, out_degree, opt.device_ptrs != 0, s))) return rc;
   uint32_t seed = seed_in;
   if (teleport == kTeleportSeed && g->relabelled)
@@ -611,26 +768,7 @@ int solve_single(nwgpu_graph* g, const uint32_t* out_degree, float* ranks, float
   }
   CK(cudaStreamSynchronize(s), "copy ranks");
   trace.mark("ranks out");
-  if (stats) {
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, g->ev0, g->ev1);
-    stats->iterations = fin.iter;
-    stats->final_error = fin.last_error;
-    stats->converged = (int32_t)fin.converged;
-    stats->device_ms = ms;
-    stats->ms_per_iter = fin.iter ? ms / (double)fin.iter : 0.0;
-    stats->gteps = ms > 0 ? (double)g->nnz * (double)fin.iter / (ms * 1e6) : 0.0;
-    if (stats->errors && stats->errors_cap) {
-      uint64_t m = fin.iter < stats->errors_cap ? fin.iter : stats->errors_cap;
-      if (m > g->err_cap) m = g->err_cap;
-      if (m) {
-        CK(cudaMemcpyAsync(stats->errors, g->err_hist, m * sizeof(double), cudaMemcpyDeviceToHost, s), "copy errors");
-        CK(cudaStreamSynchronize(s), "copy errors");
-      }
-    }
-  }
-  if (fin.aborted) return fail(NWGPU_ERR_ABORTED, "solve aborted after %llu sweeps", (unsigned long long)fin.iter);
-  return NWGPU_OK;
+  return report_solve(g, fin, stats, s);
 }
 
 }  // namespace nwgpu

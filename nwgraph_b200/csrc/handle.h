@@ -11,6 +11,7 @@
 #include "ppr.h"
 #include "binned.h"
 #include "blocked.h"
+#include "resident.h"
 
 namespace nwgpu {
 
@@ -122,6 +123,8 @@ struct nwgpu_graph {
   nwgpu::BlockPlan bplan;
   bool             blocked_off = false;  // this solve's degrees failed the blocked sweep's check: binned sweep
   bool             cg_blocked = false;   // the cached loop graph runs the blocked sweep
+  // One launch per solve for small graphs (plain and single-seed solves), looked at by the first such solve.
+  nwgpu::ResidentPlan resident;
   int          finish_grid = 1;  // finishing-kernel CTAs
   uint64_t     device_bytes = 0;
 
@@ -139,6 +142,7 @@ struct nwgpu_graph {
   double*       err_hist = nullptr;
   uint32_t      err_cap = 4096;
   nwgpu::PrState* h_st = nullptr;     // pinned mirror of *st
+  nwgpu::PrState* d_hst = nullptr;    // its device address
   unsigned int* h_abort = nullptr;  // mapped pinned abort word
   unsigned int* d_abort = nullptr;
   cudaEvent_t   ev0 = nullptr, ev1 = nullptr;
@@ -160,6 +164,7 @@ struct nwgpu_graph {
     wpr.release(stream);
     plan.release(stream);
     bplan.release(stream);
+    resident.release(stream);
     if (cg_exec) cudaGraphExecDestroy(cg_exec);
     if (cg) cudaGraphDestroy(cg);
     void* dev_ptrs[] = {g.row_ptr, g.col, g.w, g.perm, g.inv, g.emap, tiling.tile_row, tiling.tile_nnz, rank, contrib[0],
