@@ -11,6 +11,10 @@ constexpr uint32_t kChunk = 1024;    // entries per long-row chunk (one warp)
 constexpr uint32_t kBin0Rows = 2;    // bin-0 rows per warp: 2 (half a warp each) or 1 (a whole warp)
 constexpr int      kNumBins = 8;     // warp per row, then G = 32, 16, 8, 4, 2, 1, empty
 
+// Plans of at most this many chunks are finished by the sweep's last CTA.
+constexpr uint32_t kFuseChunks = 32768;
+constexpr int      kLoopSweeps = 3;  // of such a plan, per round of the device-side loop
+
 struct BinnedArgs {
   SweepArgs       sw;                     // row_ptr / col / vectors / state / loop control
   uint32_t        long_row;               // rows longer than this are chunked (> 128)
@@ -19,6 +23,7 @@ struct BinnedArgs {
   uint32_t        num_long_rows;          // rows [0, num_long_rows) are chunked
   uint32_t        num_big_rows;           // rows [0, num_big_rows) have more than 32 chunks
   uint32_t        num_chunks;
+  uint32_t        fused;                  // the sweep's last CTA finishes the long rows and the sweep (kFuseChunks)
   const uint32_t* row_first_chunk;        // num_long_rows + 1
   const uint32_t* chunk_row;              // num_chunks
   float*          chunk_part;             // num_chunks partial sums
@@ -50,7 +55,7 @@ int         binned_finish_grid(const BinnedArgs& a);
 // mode: SweepMode. The weighted and adjoint sweeps always use the hot shape
 // (sweep_grid = binned_sweep_grid(sms, true)).
 cudaError_t launch_binned_sweep(const BinnedArgs& a, bool hot, int mode, int sweep_grid, int finish_grid, cudaStream_t s);
-// finish_node (optional): the finishing kernel's node, the body's last.
+// finish_node (optional): the body's last node (the finishing kernel's, or the sweep's where it is fused).
 cudaError_t add_binned_nodes(cudaGraph_t body, const BinnedArgs& a, bool hot, int mode, int sweep_grid, int finish_grid,
                              cudaGraphNode_t* finish_node = nullptr);
 
