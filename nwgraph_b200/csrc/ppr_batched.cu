@@ -558,17 +558,25 @@ __global__ void __launch_bounds__(256) ppr_finish_kernel(const PprArgs a) {
   if (a.use_cond && !done && done_iters < st->chunk_end) cudaGraphSetConditional(a.cond, 1u);
 }
 
-// rank(i, c) = [i == seed_c], contrib = rank / deg.
+// rank(i, c) = [i == seed_c], contrib = rank / deg; four columns per thread.
 template <int K>
 __global__ void ppr_init_kernel(const PprArgs a, uint64_t n) {
-  const uint64_t total = n * K;
-  const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+  constexpr uint32_t C4 = K / 4;
+  const uint64_t     total = n * C4;
+  const uint64_t     stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < total; x += stride) {
-    const uint32_t i = (uint32_t)(x / K);
-    const int      c = (int)(x % K);
-    const float    r = (a.seeds[c] == i) ? 1.0f : 0.0f;
-    a.rank[x] = r;
-    a.contrib0[x] = r / (float)a.deg[i];
+    const uint32_t i = (uint32_t)(x / C4);
+    const int      c = (int)(x % C4) * 4;
+    const float    dg = (float)__ldg(a.deg + i), none = 0.f / dg, one = 1.f / dg;
+    float          r[4], z[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const bool is_seed = __ldg(a.seeds + c + q) == i;
+      r[q] = is_seed ? 1.0f : 0.0f;
+      z[q] = is_seed ? one : none;
+    }
+    __stcs(reinterpret_cast<float4*>(a.rank) + x, make_float4(r[0], r[1], r[2], r[3]));
+    reinterpret_cast<float4*>(a.contrib0)[x] = make_float4(z[0], z[1], z[2], z[3]);
   }
 }
 
@@ -592,17 +600,22 @@ __global__ void ppr_winit_kernel(const PprArgs a, const float* __restrict__ t_in
   }
 }
 
+// The streaming moves below take a matrix element per thread, K = 2^lk slots
+// per row: a 64-bit division by a run-time width per element held them below
+// the copy rate (RMAT scale 22, 64 columns, both moves of a narrowing: output
+// 1.43 to 1.16 ms, repack 0.73 to 0.43; the start, four columns per thread,
+// 0.90 to 0.53).
+
 // out[i * k + c] = rank[perm[i] * K + c] for c < k (input order, unpadded).
 template <int K>
 __global__ void ppr_output_kernel(const float* __restrict__ rank, const uint32_t* __restrict__ perm, uint64_t n,
                                   uint32_t k, float* __restrict__ out) {
-  const uint64_t total = n * k;
+  const uint64_t total = n * K;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < total; x += stride) {
-    const uint64_t i = x / k;
-    const uint32_t c = (uint32_t)(x % k);
-    const uint64_t src = perm ? perm[i] : i;
-    out[x] = rank[src * K + c];
+    const uint64_t i = x / K;
+    const uint32_t c = (uint32_t)(x % K);
+    if (c < k) out[i * k + c] = __ldcs(rank + (perm ? (uint64_t)__ldg(perm + i) : i) * K + c);
   }
 }
 
@@ -611,13 +624,13 @@ __global__ void ppr_output_kernel(const float* __restrict__ rank, const uint32_t
 // on it), so moving the running columns into a narrower matrix changes no
 // column's values.
 __global__ void ppr_repack_kernel(const float* __restrict__ src, float* __restrict__ dst, uint64_t n, uint32_t K_from,
-                                  uint32_t K_to, const uint32_t* __restrict__ map, uint32_t nact) {
-  const uint64_t total = n * K_to;
+                                  int lk_to, const uint32_t* __restrict__ map, uint32_t nact) {
+  const uint64_t total = n << lk_to;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < total; x += stride) {
-    const uint64_t i = x / K_to;
-    const uint32_t j = (uint32_t)(x % K_to);
-    dst[x] = j < nact ? src[i * K_from + map[j]] : 0.f;
+    const uint64_t i = x >> lk_to;
+    const uint32_t j = (uint32_t)x & ((1u << lk_to) - 1u);
+    dst[x] = j < nact ? src[i * K_from + __ldg(map + j)] : 0.f;
   }
 }
 
@@ -645,14 +658,14 @@ __global__ void ppr_repack_cols_kernel(PprArgs a, uint32_t K_to, const uint32_t*
 }
 
 __global__ void ppr_output_slots_kernel(const float* __restrict__ rank, const uint32_t* __restrict__ perm, uint64_t n,
-                                        uint32_t K, const uint32_t* __restrict__ slot_orig, uint32_t k,
+                                        int lk, const uint32_t* __restrict__ slot_orig, uint32_t k,
                                         float* __restrict__ out) {
-  const uint64_t total = n * K;
+  const uint64_t total = n << lk;
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < total; x += stride) {
-    const uint64_t i = x / K;
-    const uint32_t j = (uint32_t)(x % K), c = slot_orig[j];
-    if (c < k) out[i * k + c] = rank[(perm ? (uint64_t)perm[i] : i) * K + j];
+    const uint64_t i = x >> lk;
+    const uint32_t j = (uint32_t)x & ((1u << lk) - 1u), c = __ldg(slot_orig + j);
+    if (c < k) out[i * k + c] = __ldcs(rank + ((perm ? (uint64_t)__ldg(perm + i) : i) << lk) + j);
   }
 }
 
@@ -699,10 +712,16 @@ cudaError_t launch_ppr_seeds(const uint32_t* seeds_in, uint32_t k, int K, const 
   return cudaGetLastError();
 }
 
+static int log2_of(int K) {
+  int l = 0;
+  while ((1 << l) < K) ++l;
+  return l;
+}
+
 cudaError_t launch_ppr_repack(const float* src, float* dst, uint64_t n, int K_from, int K_to, const uint32_t* map,
                               uint32_t nact, int sms, cudaStream_t s) {
   if (K_to <= 0 || K_to > K_from || nact > (uint32_t)K_to) return cudaErrorInvalidValue;
-  ppr_repack_kernel<<<sms * 8, 256, 0, s>>>(src, dst, n, (uint32_t)K_from, (uint32_t)K_to, map, nact);
+  ppr_repack_kernel<<<sms * 8, 256, 0, s>>>(src, dst, n, (uint32_t)K_from, log2_of(K_to), map, nact);
   return cudaGetLastError();
 }
 
@@ -714,7 +733,7 @@ cudaError_t launch_ppr_repack_cols(const PprArgs& a, int K_to, const uint32_t* m
 
 cudaError_t launch_ppr_output_slots(const float* rank, const uint32_t* perm, uint64_t n, int K, const uint32_t* slot_orig,
                                     uint32_t k, float* out, int sms, cudaStream_t s) {
-  ppr_output_slots_kernel<<<sms * 8, 256, 0, s>>>(rank, perm, n, (uint32_t)K, slot_orig, k, out);
+  ppr_output_slots_kernel<<<sms * 8, 256, 0, s>>>(rank, perm, n, log2_of(K), slot_orig, k, out);
   return cudaGetLastError();
 }
 
