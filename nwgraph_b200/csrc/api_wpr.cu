@@ -28,6 +28,9 @@ void WprBuffers::release(cudaStream_t s) {
   void* ptrs[] = {t.row_ptr, t.col, t.w, t.fwd, t.s, t.erow, vbase, vaux, r_int, stage, stage2, res, gw, basis, w, vneg,
                   part, dout, f, q};
   for (void* p : ptrs) pool_free(p, s);
+  if (h_dots[0]) cudaStreamSynchronize(s);  // no reduction may still write the blocks when they are reused
+  for (double* h : h_dots)
+    if (h) host_block_put(h);
   tplan.release(s);
   *this = WprBuffers();
 }
@@ -135,7 +138,12 @@ int ensure_gmres(nwgpu_graph* g) {
   CK(dalloc(g, &b.w, n), "cudaMalloc(gmres work)");
   CK(dalloc(g, &b.vneg, n), "cudaMalloc(gmres -d/s)");
   CK(dalloc(g, &b.part, (uint64_t)vg.blocks * (kGmresRestart + 1)), "cudaMalloc(gmres partials)");
-  CK(dalloc(g, &b.dout, (uint64_t)kGmresRestart + 2), "cudaMalloc(gmres dots)");
+  CK(dalloc(g, &b.dout, 2 * ((uint64_t)kGmresMaxBasis + 1)), "cudaMalloc(gmres dots)");
+  static_assert((kGmresRestart + 1) * sizeof(double) <= kHostBlock, "a reduction fits a host block");
+  for (int i = 0; i < 2; ++i) {
+    CK(host_block_get((void**)&b.h_dots[i]), "cudaHostAlloc(gmres dots)");
+    CK(cudaHostGetDevicePointer((void**)&b.d_hdots[i], b.h_dots[i], 0), "cudaHostGetDevicePointer(gmres dots)");
+  }
   return NWGPU_OK;
 }
 
@@ -156,12 +164,6 @@ int apply_adjoint_op(nwgpu_graph* g, const SweepArgs& proto, const float* v, flo
   return NWGPU_OK;
 }
 
-int read_doubles(const double* d, double* h, int count, cudaStream_t s) {
-  CK(cudaMemcpyAsync(h, d, (size_t)count * sizeof(double), cudaMemcpyDeviceToHost, s), "copy reduction");
-  CK(cudaStreamSynchronize(s), "reduction");
-  return NWGPU_OK;
-}
-
 // Restarted GMRES for A x = c (c = vbase, internal order), x in/out (x0 on
 // entry). Stops when the L1 norm of the true residual c - A x, evaluated in
 // FP64 at the start of each cycle, is below thr, or after max_ops operator
@@ -174,8 +176,11 @@ int gmres_adjoint(nwgpu_graph* g, const SweepArgs& proto, const float* c, float*
   const int      m = kGmresRestart;
   auto           V = [&](int i) { return b.basis + (uint64_t)i * b.ld; };
   double         H[kGmresRestart + 1][kGmresRestart], cs[kGmresRestart], sn[kGmresRestart], gv[kGmresRestart + 1];
-  double         h[kGmresRestart + 2];
   float          coef[kGmresMaxBasis];
+  // the two sets of dots an iteration takes, and where the host reads them once the stream is idle
+  double* const          d1 = b.dout;
+  double* const          d2 = b.dout + kGmresMaxBasis + 1;
+  const volatile double *h1 = b.h_dots[0], *h2 = b.h_dots[1];
   *ops = 0;
   *converged = false;
   int rc;
@@ -183,20 +188,20 @@ int gmres_adjoint(nwgpu_graph* g, const SweepArgs& proto, const float* c, float*
     // r = c - A x, its L1 norm (the fixed-point iteration's L1 change) and 2-norm
     if ((rc = apply_adjoint_op(g, proto, x, b.w, s))) return rc;
     ++*ops;
-    CK(launch_vec_axpby(1.f, c, 0.f, V(0), n, vg, b.part, nullptr, s), "residual");
-    CK(launch_vec_axpby(-1.f, b.w, 1.f, V(0), n, vg, b.part, b.dout, s), "residual");
-    CK(launch_vec_dots(V(0), b.ld, 1, V(0), n, vg, b.part, b.dout + 1, s), "residual norm");
-    if ((rc = read_doubles(b.dout, h, 2, s))) return rc;
-    *res_l1 = h[0];
-    if (h[0] < thr) {
+    CK(launch_vec_axpby(1.f, c, 0.f, V(0), n, vg, b.part, nullptr, nullptr, s), "residual");
+    CK(launch_vec_axpby(-1.f, b.w, 1.f, V(0), n, vg, b.part, d1, b.d_hdots[0], s), "residual");
+    CK(launch_vec_dots(V(0), b.ld, 1, V(0), n, vg, b.part, d2, b.d_hdots[1], s), "residual norm");
+    CK(cudaStreamSynchronize(s), "residual");
+    *res_l1 = h1[0];
+    if (h1[0] < thr) {
       *converged = true;
       return NWGPU_OK;
     }
     if (*ops >= max_ops) return NWGPU_OK;
-    const double beta = sqrt(h[1]);
+    const double beta = sqrt(h2[0]);
     if (!(beta > 0.0)) return NWGPU_OK;
-    const double l1_per_l2 = h[0] / beta;  // how the L1 norm scales with the 2-norm this cycle
-    CK(launch_vec_axpby((float)(1.0 / beta), V(0), 0.f, V(0), n, vg, b.part, nullptr, s), "normalise");
+    const double l1_per_l2 = *res_l1 / beta;  // how the L1 norm scales with the 2-norm this cycle
+    CK(launch_vec_axpby((float)(1.0 / beta), V(0), 0.f, V(0), n, vg, b.part, nullptr, nullptr, s), "normalise");
     for (int i = 0; i <= m; ++i) gv[i] = 0.0;
     gv[0] = beta;
     int k = 0;  // basis vectors used this cycle
@@ -205,23 +210,22 @@ int gmres_adjoint(nwgpu_graph* g, const SweepArgs& proto, const float* c, float*
       ++*ops;
       // classical Gram-Schmidt, twice: h1 = V^T w; w' = w - V h1 with h2 = V^T w'
       // and |w'|^2 in the same pass; the new vector (w' - V h2) / |w' - V h2|,
-      // whose norm is sqrt(|w'|^2 - |h2|^2)
+      // whose norm is sqrt(|w'|^2 - |h2|^2). The coefficients stay on the device,
+      // so all of it is queued at once and the host waits once per iteration, for
+      // its copies of h1 and h2 (a wait after each set of dots took 25 us more).
       double hj[kGmresRestart + 1] = {0.0};
-      CK(launch_vec_dots(V(0), b.ld, j + 1, b.w, n, vg, b.part, b.dout, s), "Gram-Schmidt dots");
-      if ((rc = read_doubles(b.dout, h, j + 1, s))) return rc;
-      for (int i = 0; i <= j; ++i) {
-        hj[i] = h[i];
-        coef[i] = (float)h[i];
-      }
-      CK(launch_vec_update(b.w, b.w, V(0), b.ld, j + 1, coef, 1.f, n, vg, b.part, b.dout, s), "Gram-Schmidt update");
-      if ((rc = read_doubles(b.dout, h, j + 2, s))) return rc;
+      CK(launch_vec_dots(V(0), b.ld, j + 1, b.w, n, vg, b.part, d1, b.d_hdots[0], s), "Gram-Schmidt dots");
+      CK(launch_vec_project(b.w, b.w, V(0), b.ld, j + 1, d1, 0.0, n, vg, b.part, d2, b.d_hdots[1], s), "Gram-Schmidt update");
+      CK(launch_vec_project(b.w, V(j + 1), V(0), b.ld, j + 1, d2, 1e-30 * beta, n, vg, b.part, nullptr, nullptr, s),
+         "new basis vector");
+      CK(cudaStreamSynchronize(s), "Gram-Schmidt");
       double h2sq = 0.0;
       for (int i = 0; i <= j; ++i) {
-        hj[i] += h[i];
-        coef[i] = (float)h[i];
-        h2sq += h[i] * h[i];
+        hj[i] = h1[i];
+        hj[i] += h2[i];
+        h2sq += h2[i] * h2[i];
       }
-      const double nrm2 = h[j + 1] - h2sq;
+      const double nrm2 = h2[j + 1] - h2sq;
       hj[j + 1] = nrm2 > 0.0 ? sqrt(nrm2) : 0.0;
       // apply the previous rotations, then a new one that zeroes hj[j + 1]
       for (int i = 0; i < j; ++i) {
@@ -239,9 +243,6 @@ int gmres_adjoint(nwgpu_graph* g, const SweepArgs& proto, const float* c, float*
       for (int i = 0; i <= j; ++i) H[i][j] = hj[i];
       k = j + 1;
       const bool breakdown = !(hn > 1e-30 * beta);
-      if (!breakdown)
-        CK(launch_vec_update(b.w, V(j + 1), V(0), b.ld, j + 1, coef, (float)(1.0 / hn), n, vg, b.part, nullptr, s),
-           "new basis vector");
       // estimated L1 residual: the 2-norm estimate |g_{j+1}| scaled like this cycle's start
       if (breakdown || fabs(gv[j + 1]) * l1_per_l2 < 0.5 * thr || *ops >= max_ops) break;
     }
@@ -253,7 +254,7 @@ int gmres_adjoint(nwgpu_graph* g, const SweepArgs& proto, const float* c, float*
       y[i] = H[i][i] != 0.0 ? t / H[i][i] : 0.0;
     }
     for (int i = 0; i < k; ++i) coef[i] = (float)-y[i];
-    CK(launch_vec_update(x, x, V(0), b.ld, k, coef, 1.f, n, vg, b.part, nullptr, s), "update solution");
+    CK(launch_vec_update(x, x, V(0), b.ld, k, coef, 1.f, n, vg, b.part, s), "update solution");
   }
 }
 

@@ -220,16 +220,22 @@ struct VecGrid {
 };
 VecGrid     vec_grid(uint64_t n, int sms);
 // out[0..nv) = V_i . x for the nv (1..kGmresMaxBasis) vectors of V (stride
-// ld), out[nv] = x . x; part: blocks * (nv + 1) doubles
+// ld), out[nv] = x . x; part: blocks * (nv + 1) doubles; host_out (here and
+// below): mapped host memory that gets the same values, or null
 cudaError_t launch_vec_dots(const float* V, uint64_t ld, int nv, const float* x, uint64_t n, const VecGrid& vg,
-                            double* part, double* out, cudaStream_t st);
-// y = scale * (x - sum_i coef[i] V_i) (x and y may alias); with out: the dots
-// of the V_i with y, and y . y, as launch_vec_dots writes them
+                            double* part, double* out, double* host_out, cudaStream_t st);
+// y = x - sum_i dots[i] V_i (x and y may alias), dots on the device. With out:
+// the dots of the V_i with y, and y . y, as launch_vec_dots writes them.
+// Without: y scaled by 1 / |y| = 1 / sqrt(dots[nv] - sum dots[i]^2) where that
+// norm is above least, by 0 elsewhere.
+cudaError_t launch_vec_project(const float* x, float* y, const float* V, uint64_t ld, int nv, const double* dots, double least,
+                               uint64_t n, const VecGrid& vg, double* part, double* out, double* host_out, cudaStream_t st);
+// y = scale * (x - sum_i coef[i] V_i) (x and y may alias)
 cudaError_t launch_vec_update(const float* x, float* y, const float* V, uint64_t ld, int nv, const float* coef, float scale,
-                              uint64_t n, const VecGrid& vg, double* part, double* out, cudaStream_t st);
+                              uint64_t n, const VecGrid& vg, double* part, cudaStream_t st);
 // y = alpha x + beta y; with l1_out: ||y||_1 after the update
 cudaError_t launch_vec_axpby(float alpha, const float* x, float beta, float* y, uint64_t n, const VecGrid& vg,
-                             double* part, double* l1_out, cudaStream_t st);
+                             double* part, double* l1_out, double* host_out, cudaStream_t st);
 cudaError_t launch_neg_dinv(const float* s, uint64_t n, float damping, float* vaux, int sms, cudaStream_t st);
 cudaError_t launch_op_state(PrState* st, cudaStream_t s);
 

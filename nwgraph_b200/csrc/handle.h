@@ -61,7 +61,9 @@ struct WprBuffers {
   float*     w = nullptr;
   float*     vneg = nullptr;
   double*    part = nullptr;
-  double*    dout = nullptr;
+  double*    dout = nullptr;     // two sets of kGmresMaxBasis + 1
+  double*    h_dots[2] = {nullptr, nullptr};  // mapped host blocks the reductions also write, and their device addresses
+  double*    d_hdots[2] = {nullptr, nullptr};
   float*     f = nullptr;        // n: dL/dw factors d r_j / s_j
   float*     q = nullptr;        // n: dL/dw offsets q_j
   void       release(cudaStream_t s);

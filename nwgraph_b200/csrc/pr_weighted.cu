@@ -139,18 +139,30 @@ __device__ __forceinline__ double block_sum(double v, double* s_red) {
   return t;  // valid in thread 0
 }
 
-// out[i] = sum_b part[b * nv + i], lane-strided over the blocks, fixed tree.
-__global__ void vec_reduce_kernel(const double* __restrict__ part, int nblocks, int nv, double* __restrict__ out) {
+// out[i] = sum_b part[b * nv + i], lane-strided over the blocks, fixed tree;
+// host_out (mapped host memory, or null): the same values.
+__global__ void vec_reduce_kernel(const double* __restrict__ part, int nblocks, int nv, double* __restrict__ out,
+                                  double* __restrict__ host_out) {
   const int i = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= nv) return;
   double acc = 0.0;
   for (int b = lane; b < nblocks; b += 32) acc += part[(uint64_t)b * nv + i];
   acc = warp_sum_lane0(acc);
-  if (lane == 0) out[i] = acc;
+  if (lane == 0) {
+    out[i] = acc;
+    if (host_out) host_out[i] = acc;
+  }
 }
 
+// Coefficients of an update: c and scale by value; or, with dots, on the device
+// from an earlier reduction: c = dots[0..nv), and with `unit` the scale that
+// makes the result a unit vector, 1 / sqrt(dots[nv] - sum dots[i]^2) (0 when
+// that is not above least), rounded as the host would round them.
 struct VecCoeffs {
-  float c[kGmresMaxBasis];
+  float         c[kGmresMaxBasis];
+  const double* dots;
+  int           unit;
+  double        least;
 };
 
 // One pass over the nv (<= NV) basis vectors of V (stride ld) and x:
@@ -166,6 +178,20 @@ __global__ void __launch_bounds__(kVecThreads) vec_gs_kernel(const float* x, flo
                                                              uint64_t n, uint64_t chunk, double* __restrict__ part) {
   __shared__ double s_red[kVecThreads / 32][NV + 1];
   const uint64_t    k0 = (uint64_t)blockIdx.x * chunk, k1 = min(n, k0 + chunk);
+  float             c[NV];
+  if constexpr (UPDATE) {
+#pragma unroll
+    for (int i = 0; i < NV; ++i) c[i] = a.dots ? (i < nv ? (float)__ldg(a.dots + i) : 0.f) : a.c[i];
+    if (a.dots && a.unit) {
+      double h2 = 0.0;
+      for (int i = 0; i < nv; ++i) {
+        const double h = __ldg(a.dots + i);
+        h2 = __dadd_rn(h2, __dmul_rn(h, h));
+      }
+      const double nrm2 = __dadd_rn(__ldg(a.dots + nv), -h2), hn = nrm2 > 0.0 ? sqrt(nrm2) : 0.0;
+      scale = hn > a.least ? (float)(1.0 / hn) : 0.f;
+    }
+  }
   float             acc[NV + 1];
 #pragma unroll
   for (int i = 0; i <= NV; ++i) acc[i] = 0.f;
@@ -176,7 +202,7 @@ __global__ void __launch_bounds__(kVecThreads) vec_gs_kernel(const float* x, flo
     float v = x[k];
     if constexpr (UPDATE) {
 #pragma unroll
-      for (int i = 0; i < NV; ++i) v = fmaf(-a.c[i], vv[i], v);
+      for (int i = 0; i < NV; ++i) v = fmaf(-c[i], vv[i], v);
       v *= scale;
       y[k] = v;
     }
@@ -257,34 +283,46 @@ VecGrid vec_grid(uint64_t n, int sms) {
 
 // out[0..nv) = V_i . x, out[nv] = x . x
 cudaError_t launch_vec_dots(const float* V, uint64_t ld, int nv, const float* x, uint64_t n, const VecGrid& vg,
-                            double* part, double* out, cudaStream_t st) {
+                            double* part, double* out, double* host_out, cudaStream_t st) {
   if (nv < 1 || nv > kGmresMaxBasis) return cudaErrorInvalidValue;
   VecCoeffs   a = {};
   cudaError_t e = launch_gs<false, true>(x, nullptr, V, ld, nv, a, 1.f, n, vg, part, st);
   if (e != cudaSuccess) return e;
-  vec_reduce_kernel<<<(nv + 1 + 7) / 8, 256, 0, st>>>(part, vg.blocks, nv + 1, out);
+  vec_reduce_kernel<<<(nv + 1 + 7) / 8, 256, 0, st>>>(part, vg.blocks, nv + 1, out, host_out);
   return cudaGetLastError();
 }
 
-// y = scale * (x - sum_i coef[i] V_i); with out: out[0..nv) = V_i . y, out[nv] = y . y
+// y = x - sum_i dots[i] V_i on the device's coefficients; with out: the dots of
+// y, as launch_vec_dots writes them; without: y scaled to a unit vector
+cudaError_t launch_vec_project(const float* x, float* y, const float* V, uint64_t ld, int nv, const double* dots, double least,
+                               uint64_t n, const VecGrid& vg, double* part, double* out, double* host_out, cudaStream_t st) {
+  if (nv < 1 || nv > kGmresMaxBasis) return cudaErrorInvalidValue;
+  VecCoeffs a = {};
+  a.dots = dots;
+  a.unit = out ? 0 : 1;
+  a.least = least;
+  if (!out) return launch_gs<true, false>(x, y, V, ld, nv, a, 1.f, n, vg, part, st);
+  cudaError_t e = launch_gs<true, true>(x, y, V, ld, nv, a, 1.f, n, vg, part, st);
+  if (e != cudaSuccess) return e;
+  vec_reduce_kernel<<<(nv + 1 + 7) / 8, 256, 0, st>>>(part, vg.blocks, nv + 1, out, host_out);
+  return cudaGetLastError();
+}
+
+// y = scale * (x - sum_i coef[i] V_i)
 cudaError_t launch_vec_update(const float* x, float* y, const float* V, uint64_t ld, int nv, const float* coef, float scale,
-                              uint64_t n, const VecGrid& vg, double* part, double* out, cudaStream_t st) {
+                              uint64_t n, const VecGrid& vg, double* part, cudaStream_t st) {
   if (nv < 1 || nv > kGmresMaxBasis) return cudaErrorInvalidValue;
   VecCoeffs a = {};
   for (int i = 0; i < nv; ++i) a.c[i] = coef[i];
-  if (!out) return launch_gs<true, false>(x, y, V, ld, nv, a, scale, n, vg, part, st);
-  cudaError_t e = launch_gs<true, true>(x, y, V, ld, nv, a, scale, n, vg, part, st);
-  if (e != cudaSuccess) return e;
-  vec_reduce_kernel<<<(nv + 1 + 7) / 8, 256, 0, st>>>(part, vg.blocks, nv + 1, out);
-  return cudaGetLastError();
+  return launch_gs<true, false>(x, y, V, ld, nv, a, scale, n, vg, part, st);
 }
 
 cudaError_t launch_vec_axpby(float alpha, const float* x, float beta, float* y, uint64_t n, const VecGrid& vg,
-                             double* part, double* l1_out, cudaStream_t st) {
+                             double* part, double* l1_out, double* host_out, cudaStream_t st) {
   vec_axpby_kernel<<<vg.blocks, kVecThreads, 0, st>>>(alpha, x, beta, y, n, vg.chunk, l1_out ? part : nullptr);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess || !l1_out) return e;
-  vec_reduce_kernel<<<1, 256, 0, st>>>(part, vg.blocks, 1, l1_out);
+  vec_reduce_kernel<<<1, 256, 0, st>>>(part, vg.blocks, 1, l1_out, host_out);
   return cudaGetLastError();
 }
 
