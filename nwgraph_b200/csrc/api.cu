@@ -534,10 +534,34 @@ bool same_loop(const nwgpu_graph* g, const SweepArgs& y, const BinPlan* plan, in
          x.vbase == y.vbase && x.vaux == y.vaux && x.push_threshold == y.push_threshold;
 }
 
+constexpr int      kFirstLooks = 4;   // a handle's first loop: looks at the state, and sweeps launched before each
+constexpr uint64_t kFirstSweeps = 8;
+
 // Runs the sweep loop from the state already on the device; fills fin.
 int run_sweeps(nwgpu_graph* g, const SweepArgs& a, uint32_t launch, uint64_t max_iters, cudaStream_t s, PrState* fin,
                const BinPlan* plan, int mode) {
   if (launch == NWGPU_LAUNCH_GRAPH) {
+    // A handle's first loop is launched sweep by sweep, a few per look at the state: a graph that runs once (the
+    // reference's one-shot call) costs its instantiation and destruction, 190 us each, where a sweep's launch costs 3
+    // and one after the last sweep returns at once. A long first loop goes on with the graph.
+    if (plan && !g->looped && !g->cg_exec && !use_blocked(g, plan, mode)) {
+      const BinnedArgs ba = make_binned_args(g, *plan, a, mode);
+      uint64_t         launched = 0;
+      for (int look = 0; look < kFirstLooks && launched < max_iters; ++look) {
+        const uint64_t batch = std::min<uint64_t>(kFirstSweeps, max_iters - launched);
+        for (uint64_t b = 0; b < batch; ++b)
+          CK(launch_binned_sweep(ba, plan->hot, mode, binned_grid(g, *plan, mode), plan->finish_grid, s), "pr_binned_sweep");
+        launched += batch;
+        CK(cudaMemcpyAsync(g->h_st, g->st, sizeof(PrState), cudaMemcpyDeviceToHost, s), "copy state");
+        CK(cudaStreamSynchronize(s), "sweep loop");
+        if (g->h_st->done) break;
+      }
+      g->looped = launched > 0;
+      if (g->h_st->done) {
+        *fin = *g->h_st;
+        return fin->fault ? fail(NWGPU_ERR_CUDA, "a bounded device wait gave up (fault word %u)", fin->fault) : NWGPU_OK;
+      }
+    }
     if (!g->cg_exec || !same_loop(g, a, plan, mode)) {
       int rc = build_loop_graph(g, a, plan, mode);
       if (rc) return rc;

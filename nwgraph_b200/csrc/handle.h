@@ -149,7 +149,8 @@ struct nwgpu_graph {
   unsigned int* d_abort = nullptr;
   cudaEvent_t   ev0 = nullptr, ev1 = nullptr;
 
-  // CUDA graph of the sweep loop (arm node -> while node { sweep; finish }).
+  // CUDA graph of the sweep loop (arm node -> while node { sweep; finish }), built by the second loop.
+  bool            looped = false;  // a first loop has run
   cudaGraph_t     cg = nullptr;
   cudaGraphExec_t cg_exec = nullptr;
   nwgpu::SweepArgs cg_args{};  // arguments baked into cg_exec

@@ -36,6 +36,17 @@ def test_launch_modes_and_shapes(gpu, monkeypatch):
         assert np.array_equal(a, b)
 
 
+@pytest.mark.parametrize("its", [1, 8, 9, 32, 33, 70])
+def test_first_loop_then_graph(gpu, its):
+    """A handle's first loop launches its sweeps itself, and goes on with the loop graph after 32."""
+    rp, col, deg = _graph()
+    a, b = np.empty(len(deg), np.float32), np.empty(len(deg), np.float32)
+    with Graph(rp, col) as g:
+        s0 = g.page_rank(deg, a, 0.85, -1.0, its, record_errors=True)
+        s1 = g.page_rank(deg, b, 0.85, -1.0, its, record_errors=True)
+    assert np.array_equal(a, b) and s0.iterations == s1.iterations == its and np.array_equal(s0.errors, s1.errors)
+
+
 def test_both_sides_of_the_chunk_limit(gpu, monkeypatch):
     """Rows of 257 to 300 entries, one or two chunks each: 2 x 16,384 chunks are finished by the last CTA, two more
     are not. The ranks may depend on neither."""
