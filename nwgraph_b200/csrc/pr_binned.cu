@@ -163,15 +163,6 @@ __device__ __forceinline__ double binned_epilogue(const BinnedArgs& a, float* __
   return binned_update<MODE>(a, cout, r, z, load_row_in<MODE>(a, r), pol);
 }
 
-// One term of a row sum: the gathered contribution, times the entry's weight
-// in the weighted and adjoint modes.
-template <bool HOT, int MODE>
-__device__ __forceinline__ float term(const BinnedArgs& a, const Src& src, uint32_t id, uint32_t k) {
-  const float c = gather_one<HOT, MODE>(src, id);
-  if constexpr (MODE == kModePlain || MODE == kModeResidual || MODE == kModeRagged) return c;
-  else return ld_stream(a.sw.w + k) * c;
-}
-
 // Rows without entries: four rows per lane.
 template <int MODE>
 __device__ __forceinline__ double empty_rows(const BinnedArgs& a, float* __restrict__ cout, uint32_t row0,
@@ -241,24 +232,47 @@ __device__ __forceinline__ void load_window(const uint32_t* __restrict__ col, ui
   }
 }
 
-// The window's terms: the gathered contributions of its ids, times the
-// entries' weights in the weighted and adjoint modes. The weights lie beside
-// the ids (same CSR order) and load as the same words; they are not held ahead
-// in registers like the ids, but the step before asks L2 for their lines
-// (prefetch_weights), so that they arrive no later than the gathers.
+// The terms of a lane's 8 entries: the gathered contributions and, in the
+// weighted and adjoint modes, the entries' weights, which lie beside the ids
+// (same CSR order) and load as the same words. They are multiplied only when
+// they are added (term_of), after the next step's ids have been asked for:
+// a product taken at once waits for both loads first, and a step then costs
+// the latencies of its gathers and of the next ids one after the other.
+template <int MODE>
+constexpr bool kWeightedMode = MODE == kModeWeighted || MODE == kModeAdjoint;
+template <bool WEIGHTED>
+struct TermsOf {
+  float c[8];
+};
+template <>
+struct TermsOf<true> {
+  float    c[8];
+  uint32_t w[8];  // the weights' bits
+  uint32_t in;    // bit q: entry q is in the window
+};
+template <int MODE>
+using Terms = TermsOf<kWeightedMode<MODE>>;
 template <bool HOT, int MODE, uint32_t L>
 __device__ __forceinline__ void window_terms(const BinnedArgs& a, const Src& src, uint32_t start, uint32_t end,
-                                             uint32_t lanei, const uint32_t (&id)[8], float (&v)[8]) {
-  if constexpr (MODE == kModeWeighted || MODE == kModeAdjoint) {
-    uint32_t wv[8];
-    load_window<L>(reinterpret_cast<const uint32_t*>(a.sw.w), start, end, lanei, wv);
+                                             uint32_t lanei, const uint32_t (&id)[8], Terms<MODE>& t) {
+  if constexpr (kWeightedMode<MODE>) {
+    load_window<L>(reinterpret_cast<const uint32_t*>(a.sw.w), start, end, lanei, t.w);
+    t.in = 0u;
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      v[q] = (window_entry<L>(start, lanei, q) < end) ? __uint_as_float(wv[q]) * gather_one<HOT, MODE>(src, id[q]) : 0.f;
+    for (int q = 0; q < 8; ++q) {
+      const bool in = window_entry<L>(start, lanei, q) < end;
+      t.c[q] = in ? gather_one<HOT, MODE>(src, id[q]) : 0.f;
+      t.in |= in ? 1u << q : 0u;
+    }
   } else {
 #pragma unroll
-    for (int q = 0; q < 8; ++q) v[q] = (window_entry<L>(start, lanei, q) < end) ? gather_one<HOT, MODE>(src, id[q]) : 0.f;
+    for (int q = 0; q < 8; ++q) t.c[q] = (window_entry<L>(start, lanei, q) < end) ? gather_one<HOT, MODE>(src, id[q]) : 0.f;
   }
+}
+template <int MODE>
+__device__ __forceinline__ float term_of(const Terms<MODE>& t, int q) {
+  if constexpr (kWeightedMode<MODE>) return (t.in >> q) & 1u ? __fmul_rn(__uint_as_float(t.w[q]), t.c[q]) : 0.f;
+  else return t.c[q];
 }
 // One line per lane; the window's last line may be its first entry's alone.
 template <int MODE, uint32_t L>
@@ -320,8 +334,8 @@ __device__ __forceinline__ double range_bin(const BinnedArgs& a, const Src& src,
   };
 #pragma unroll 1
   for (;;) {
-    float v[U];
-    window_terms<HOT, MODE, STEP>(a, src, base, k1, (uint32_t)lane, id, v);
+    Terms<MODE> t;
+    window_terms<HOT, MODE, STEP>(a, src, base, k1, (uint32_t)lane, id, t);
     if (pending) {
       finish();
       pending = false;
@@ -334,7 +348,7 @@ __device__ __forceinline__ double range_bin(const BinnedArgs& a, const Src& src,
     load_window<STEP>(a.sw.col, nbase, nend, (uint32_t)lane, id);
     prefetch_weights<MODE, STEP>(a, nbase, nend, (uint32_t)lane);
 #pragma unroll
-    for (int q = 0; q < U; ++q) acc += v[q];
+    for (int q = 0; q < U; ++q) acc += term_of<MODE>(t, q);
     if (!more) {
       pending = true;
       acc_done = acc;
@@ -401,8 +415,8 @@ __device__ __forceinline__ double pair_bin(const BinnedArgs& a, const Src& src, 
   };
 #pragma unroll 1
   for (;;) {
-    float v[U];
-    window_terms<HOT, MODE, STEP>(a, src, base, k1, sub, id, v);
+    Terms<MODE> t;
+    window_terms<HOT, MODE, STEP>(a, src, base, k1, sub, id, t);
     if (pending) {
       finish();
       pending = false;
@@ -416,7 +430,7 @@ __device__ __forceinline__ double pair_bin(const BinnedArgs& a, const Src& src, 
     load_window<STEP>(a.sw.col, nbase, nend, sub, id);
     prefetch_weights<MODE, STEP>(a, nbase, nend, sub);
 #pragma unroll
-    for (int q = 0; q < U; ++q) acc += v[q];
+    for (int q = 0; q < U; ++q) acc += term_of<MODE>(t, q);
     if (!more) {
       pending = true;
       acc_done = acc;
@@ -506,14 +520,28 @@ __device__ __forceinline__ double group_bin(const BinnedArgs& a, const Src& src,
       const uint32_t r = rb + w * (2u * PER) + (uint32_t)h * PER + (uint32_t)lane / G;
       in[h] = (r < re_bin && sub == 0) ? load_row_in<MODE>(a, r) : no_row_in();
     }
-    float v[2][4];
+    Terms<MODE> t;  // entry q of row h: slot 4 h + q
+    if constexpr (kWeightedMode<MODE>) {
+      t.in = 0xffu;  // no entry: contribution and weight 0
 #pragma unroll
-    for (int h = 0; h < 2; ++h)
+      for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int q = 0; q < 4; ++q)
-        v[h][q] = ((uint32_t)sub + (uint32_t)q * G < len[h])
-                      ? term<HOT, MODE>(a, src, id[h][q], rs[h] + (uint32_t)sub + (uint32_t)q * G)
-                      : 0.f;
+        for (int q = 0; q < 4; ++q) {
+          const uint32_t o = (uint32_t)sub + (uint32_t)q * G;
+          t.w[4 * h + q] = 0u;
+          t.c[4 * h + q] = 0.f;
+          if (o < len[h]) {
+            t.c[4 * h + q] = gather_one<HOT, MODE>(src, id[h][q]);
+            t.w[4 * h + q] = ld_stream(reinterpret_cast<const uint32_t*>(a.sw.w) + rs[h] + o);
+          }
+        }
+    } else {
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          t.c[4 * h + q] = ((uint32_t)sub + (uint32_t)q * G < len[h]) ? gather_one<HOT, MODE>(src, id[h][q]) : 0.f;
+    }
     if (pending) finish();
     // the next unit's column ids, the bounds of the unit after it
     group_ids<G>(a, nrs, nlen, sub, id);
@@ -532,7 +560,7 @@ __device__ __forceinline__ double group_bin(const BinnedArgs& a, const Src& src,
     for (int h = 0; h < 2; ++h) {
       float acc = 0.f;
 #pragma unroll
-      for (int q = 0; q < 4; ++q) acc += v[h][q];
+      for (int q = 0; q < 4; ++q) acc += term_of<MODE>(t, 4 * h + q);
       acc_done[h] = acc;
       in_done[h] = in[h];
     }
