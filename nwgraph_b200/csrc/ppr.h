@@ -8,6 +8,8 @@ namespace nwgpu {
 
 constexpr int kPprTileItems = 512;  // merge items per tile
 constexpr int kPprThreads = 256;    // gather CTA
+// Sweeps per round of the device-side loop, whose own step costs about 5 us; sweeps after the last return at once.
+constexpr int kPprLoopSweeps = 3;
 // What a batched solve's columns are: one-hot teleports at seeds; teleport
 // vectors on a weighted graph; teleport vectors on an unweighted graph.
 constexpr int kPprSeeds = 0, kPprWeighted = 1, kPprTeleports = 2;

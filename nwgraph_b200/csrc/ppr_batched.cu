@@ -419,16 +419,19 @@ __global__ void __launch_bounds__(256) ppr_fixup_kernel(const PprArgs a) {
     float4 z[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) z[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-    for (uint32_t u = span.y; u < span.z; u += 8) {
+    const float4 e = __ldcg(reinterpret_cast<const float4*>(a.epart) + (uint64_t)span.z * P + sub);
+    for (uint32_t u = span.y; u < span.z; u += 16) {  // 16 loads in flight
+      float4 x[16];
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
-        if (u + j < span.z) {
-          const float4 x = __ldcg(part + (uint64_t)(u + j) * P);
-          z[j].x += x.x;
-          z[j].y += x.y;
-          z[j].z += x.z;
-          z[j].w += x.w;
-        }
+      for (int j = 0; j < 16; ++j)
+        x[j] = u + j < span.z ? __ldcg(part + (uint64_t)(u + j) * P) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        z[j % 8].x += x[j].x;
+        z[j % 8].y += x[j].y;
+        z[j % 8].z += x[j].z;
+        z[j % 8].w += x[j].w;
+      }
     }
     float4 t = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
@@ -438,7 +441,6 @@ __global__ void __launch_bounds__(256) ppr_fixup_kernel(const PprArgs a) {
       t.z += z[j].z;
       t.w += z[j].w;
     }
-    const float4 e = __ldcg(reinterpret_cast<const float4*>(a.epart) + (uint64_t)span.z * P + sub);
     reinterpret_cast<float4*>(cout)[(uint64_t)span.x * P + sub] = make_float4(t.x + e.x, t.y + e.y, t.z + e.z, t.w + e.w);
   }
 }
@@ -520,8 +522,15 @@ __global__ void __launch_bounds__(256) ppr_finish_kernel(const PprArgs a) {
   const unsigned long long it = *(volatile unsigned long long*)&st->iter;
   const int      lane = threadIdx.x & 31, c = blockIdx.x * 8 + (threadIdx.x >> 5);
   if (c < K && !a.col_done[c]) {  // uniform across the warp
+    // lane-strided, in order, 8 loads in flight (one at a time they were 10 us of every sweep)
     double e = 0.0;
-    for (uint32_t u = lane; u < a.epi_grid; u += 32) e += __ldcg(a.res_part + (uint64_t)u * K + c);
+    for (uint32_t u = lane; u < a.epi_grid; u += 256u) {
+      double v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = u + 32u * j < a.epi_grid ? __ldcg(a.res_part + (uint64_t)(u + 32u * j) * K + c) : 0.0;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) e += v[j];
+    }
     e = warp_sum_lane0(e);
     if (lane == 0) {
       a.col_err[c] = e;
@@ -882,7 +891,8 @@ cudaError_t build_ppr_graph(cudaGraph_t g, const PprArgs& proto, int K, int swee
   void*                args[] = {(void*)&a};
   void*                eargs[] = {(void*)&a, (void*)&n};
   cudaGraphNode_t      prev = nullptr;
-  for (int w = 0; w < 4; ++w) {
+  for (int i = 0; i < 4 * kPprLoopSweeps; ++i) {
+    const int            w = i % 4;
     cudaKernelNodeParams kp2 = {};
     kp2.func = ppr_fn(K, w, ppr_mode(a), a.few_tiles != 0);
     kp2.gridDim = ppr_grid(a, w, sweep_grid);
