@@ -550,7 +550,8 @@ def _time_port(g, deg):
 def launches_per_step(args):
     """Kernels one timed step launches: degrees to internal order (relabelled
     graphs), rank init, two per sweep (the sweep kernel and its finishing
-    kernel, on the binned and the merge-path sweep alike), the CUDA graph's
+    kernel, on the merge-path sweep and on binned plans of more than 32,768
+    long-row chunks, scale 24's among them), the CUDA graph's
     arm kernel, ranks back to input order (relabelled graphs)."""
     return SWEEPS * 2 + 1 + (1 if args.launch == "graph" else 0) + (2 if not args.no_relabel else 0)
 
