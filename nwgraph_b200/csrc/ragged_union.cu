@@ -120,14 +120,7 @@ __global__ void __launch_bounds__(256) union_chunk_kernel(UnionParts p, const ui
     const uint64_t u0 = p.voff[lo] + (uint64_t)(c - p.coff[lo]) * kUnionChunk;
     const uint64_t u1 = u0 + kUnionChunk < p.voff[lo + 1] ? u0 + kUnionChunk : p.voff[lo + 1];
     double         e = 0.0;
-    // added in order, 8 changes in flight per lane: each is a load of its row and then of the change
-    for (uint64_t u = u0 + lane; u < u1; u += 256) {
-      double v[8];
-#pragma unroll
-      for (int q = 0; q < 8; ++q) v[q] = u + 32 * q < u1 ? __ldcg(row_res + perm[u + 32 * q]) : 0.0;
-#pragma unroll
-      for (int q = 0; q < 8; ++q) e += v[q];
-    }
+    for (uint64_t u = u0 + lane; u < u1; u += 32) e += __ldcg(row_res + perm[u]);
     e = warp_sum_lane0(e);
     if (lane == 0) p.chunk_part[c] = e;
   }
