@@ -308,6 +308,13 @@ int nwgpu_abort(nwgpu_graph* g);
  * long that took. Nothing faults; the context stays usable. */
 int nwgpu_selftest_bounded_wait(uint32_t polls, uint32_t* gave_up, double* ms);
 
+/* Self-test of the engine's behaviour when memory runs out: of the calling
+ * thread's allocations of device memory or of small pinned host blocks, the
+ * one after `after` more fails, once, as if the memory were not there (the
+ * call that needed it returns NWGPU_ERR_OUT_OF_MEMORY and the handle stays
+ * usable). after < 0: none fails. */
+int nwgpu_selftest_fail_allocation(int64_t after);
+
 /* ---- Graph construction on the device ------------------------------------
  * CSR from an edge list (src[e] -> dst[e], m edges over n vertices): the
  * reference's remove_self_loops (build.hpp:404-410), uniq (:394-402) and

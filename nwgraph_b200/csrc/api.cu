@@ -207,8 +207,7 @@ uint64_t residual_parts(const nwgpu_graph* g) {
   return parts;
 }
 
-int ensure_solve_buffers(nwgpu_graph* g) {
-  if (g->solve_ready) return NWGPU_OK;
+static int alloc_solve_buffers(nwgpu_graph* g) {
   const uint64_t n = g->n, T = g->tiling.num_tiles;
   CK(dalloc(g, &g->rank, n), "cudaMalloc(rank)");
   CK(dalloc(g, &g->contrib[0], n), "cudaMalloc(contrib)");
@@ -229,8 +228,31 @@ int ensure_solve_buffers(nwgpu_graph* g) {
   CK(cudaEventCreate(&g->ev0), "cudaEventCreate");
   CK(cudaEventCreate(&g->ev1), "cudaEventCreate");
   CK(cudaStreamSynchronize(g->stream), "solve buffers");
-  g->solve_ready = true;
   return NWGPU_OK;
+}
+
+static void release_solve_buffers(nwgpu_graph* g) {
+  for (void* p : {(void*)g->rank, (void*)g->contrib[0], (void*)g->contrib[1], (void*)g->deg, (void*)g->stage_u32,
+                  (void*)g->cpart, (void*)g->epart, (void*)g->res_part, (void*)g->st, (void*)g->err_hist})
+    pool_free(p, g->stream);
+  g->rank = g->contrib[0] = g->contrib[1] = g->cpart = g->epart = nullptr;
+  g->deg = g->stage_u32 = nullptr;
+  g->res_part = g->err_hist = nullptr;
+  g->st = nullptr;
+  host_block_put(g->h_st);
+  host_block_put(g->h_abort);
+  g->h_st = g->d_hst = nullptr;
+  g->h_abort = g->d_abort = nullptr;
+  if (g->ev0) cudaEventDestroy(g->ev0);
+  if (g->ev1) cudaEventDestroy(g->ev1);
+  g->ev0 = g->ev1 = nullptr;
+}
+
+int ensure_solve_buffers(nwgpu_graph* g) {
+  if (g->solve_ready) return NWGPU_OK;
+  const int rc = all_or_none(g, [&] { return alloc_solve_buffers(g); }, [&] { release_solve_buffers(g); });
+  g->solve_ready = rc == NWGPU_OK;
+  return rc;
 }
 
 int load_degrees(nwgpu_graph* g, const uint32_t* out_degree, bool device_ptrs, cudaStream_t s) {
@@ -403,12 +425,12 @@ static int ensure_resident(nwgpu_graph* g) {
     return NWGPU_OK;
   const int      C = resident_ctas(g->n, g->nnz, g->sms);
   const uint64_t words = 2 * ((uint64_t)C + 1) + kNumResidentHubs;
-  CK(dalloc(g, &p.bounds, (uint64_t)C + 1), "cudaMalloc(resident bounds)");
-  CK(dalloc(g, &p.sync, 2), "cudaMalloc(resident counters)");
-  CK(dalloc(g, &p.part, 2 * ((uint64_t)C + 1)), "cudaMalloc(resident partials)");
   std::vector<uint32_t> h(words);
   uint32_t*             d = nullptr;
-  cudaError_t           e = pool_alloc_n(&d, words, g->stream);
+  cudaError_t           e = dalloc(g, &p.bounds, (uint64_t)C + 1);
+  if (e == cudaSuccess) e = dalloc(g, &p.sync, 2);
+  if (e == cudaSuccess) e = dalloc(g, &p.part, 2 * ((uint64_t)C + 1));
+  if (e == cudaSuccess) e = pool_alloc_n(&d, words, g->stream);
   if (e == cudaSuccess) e = launch_resident_bounds(g->g.row_ptr, g->n, g->nnz, C, p.bounds, d, g->stream);
   if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), d, words * sizeof(uint32_t), cudaMemcpyDeviceToHost, g->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
@@ -885,6 +907,12 @@ int nwgpu_selftest_bounded_wait(uint32_t polls, uint32_t* gave_up, double* ms) {
   CK(run_wait_selftest(polls, &flag, &t), "bounded-wait self-test");
   *gave_up = flag;
   *ms = t;
+  return NWGPU_OK;
+}
+
+int nwgpu_selftest_fail_allocation(int64_t after) {
+  clear_error();
+  fail_allocation(after);
   return NWGPU_OK;
 }
 

@@ -47,10 +47,8 @@ static int list_full_rows(nwgpu_graph* g, uint32_t* rows) {
   return NWGPU_OK;
 }
 
-static int ensure_ppr(nwgpu_graph* g, int K) {
-  PprBuffers& b = g->ppr;
-  if (b.K == K) return NWGPU_OK;
-  b.release(g->stream);
+static int build_ppr(nwgpu_graph* g, int K) {
+  PprBuffers&    b = g->ppr;
   const uint64_t n = g->n, nk = g->n * (uint64_t)K;
   CK(build_tiling(g->g.row_ptr, n, g->nnz, (uint32_t)kPprTileItems, &b.tiling, g->stream), "ppr tiling");
   const uint64_t T = b.tiling.num_tiles;
@@ -102,6 +100,12 @@ static int ensure_ppr(nwgpu_graph* g, int K) {
   CK(cudaStreamSynchronize(g->stream), "ppr buffers");
   b.K = K;
   return NWGPU_OK;
+}
+
+static int ensure_ppr(nwgpu_graph* g, int K) {
+  if (g->ppr.K == K) return NWGPU_OK;
+  g->ppr.release(g->stream);
+  return all_or_none(g, [&] { return build_ppr(g, K); }, [&] { g->ppr.release(g->stream); });
 }
 
 int ppr_loop(nwgpu_graph* g, const PprArgs& a, int K, uint32_t k, float* ranks_nxk, float damping, uint64_t max_iters,

@@ -24,20 +24,27 @@ using namespace nwgpu;
 
 namespace nwgpu {
 
-void WprBuffers::release(cudaStream_t s) {
-  void* ptrs[] = {t.row_ptr, t.col, t.w, t.fwd, t.s, t.erow, vbase, vaux, r_int, stage, stage2, res, gw, basis, w, vneg,
-                  part, dout, f, q};
-  for (void* p : ptrs) pool_free(p, s);
+void WprBuffers::release_gmres(cudaStream_t s) {
+  for (void* p : {(void*)basis, (void*)w, (void*)vneg, (void*)part, (void*)dout}) pool_free(p, s);
   if (h_dots[0]) cudaStreamSynchronize(s);  // no reduction may still write the blocks when they are reused
   for (double* h : h_dots)
     if (h) host_block_put(h);
+  basis = w = vneg = nullptr;
+  part = dout = nullptr;
+  for (int i = 0; i < 2; ++i) h_dots[i] = d_hdots[i] = nullptr;
+  gmres_ready = false;
+}
+
+void WprBuffers::release(cudaStream_t s) {
+  release_gmres(s);
+  void* ptrs[] = {t.row_ptr, t.col, t.w, t.fwd, t.s, t.erow, vbase, vaux, r_int, stage, stage2, res, gw, f, q};
+  for (void* p : ptrs) pool_free(p, s);
   tplan.release(s);
   *this = WprBuffers();
 }
 
-int ensure_wpr(nwgpu_graph* g) {
-  WprBuffers& b = g->wpr;
-  if (b.ready) return NWGPU_OK;
+static int build_wpr(nwgpu_graph* g) {
+  WprBuffers&    b = g->wpr;
   const uint64_t n = g->n, nnz = g->nnz;
   CK(build_transpose(g->g.row_ptr, g->g.col, g->g.w, n, nnz, g->sms, &b.t, g->stream), "out-row CSR");
   g->device_bytes += (4 * (nnz + kPad) + 2 * (n + kPad) + 1) * sizeof(uint32_t);
@@ -55,6 +62,11 @@ int ensure_wpr(nwgpu_graph* g) {
   CK(cudaStreamSynchronize(g->stream), "wpr buffers");
   b.ready = true;
   return NWGPU_OK;
+}
+
+int ensure_wpr(nwgpu_graph* g) {
+  if (g->wpr.ready) return NWGPU_OK;
+  return all_or_none(g, [&] { return build_wpr(g); }, [&] { g->wpr.release(g->stream); });
 }
 
 namespace {
@@ -128,9 +140,8 @@ int device_vector(const float* v, float* stage, uint64_t n, bool device_ptrs, cu
 constexpr int kGmresRestart = 30;
 static_assert(kGmresRestart <= kGmresMaxBasis, "more basis vectors than the update kernel takes");
 
-int ensure_gmres(nwgpu_graph* g) {
-  WprBuffers& b = g->wpr;
-  if (b.basis) return NWGPU_OK;
+int build_gmres(nwgpu_graph* g) {
+  WprBuffers&    b = g->wpr;
   const uint64_t n = g->n;
   b.ld = (n + kPad + 3) & ~3ull;
   const VecGrid vg = vec_grid(n, g->sms);
@@ -144,7 +155,13 @@ int ensure_gmres(nwgpu_graph* g) {
     CK(host_block_get((void**)&b.h_dots[i]), "cudaHostAlloc(gmres dots)");
     CK(cudaHostGetDevicePointer((void**)&b.d_hdots[i], b.h_dots[i], 0), "cudaHostGetDevicePointer(gmres dots)");
   }
+  b.gmres_ready = true;
   return NWGPU_OK;
+}
+
+int ensure_gmres(nwgpu_graph* g) {
+  if (g->wpr.gmres_ready) return NWGPU_OK;
+  return all_or_none(g, [&] { return build_gmres(g); }, [&] { g->wpr.release_gmres(g->stream); });
 }
 
 // out = A v = v - d P^T v: one adjoint sweep over the out-row CSR with
@@ -372,6 +389,23 @@ __global__ void spmv_fill_kernel(float* __restrict__ p, uint64_t n, float v) {
   const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) p[i] = v;
 }
+
+static int ensure_spmv(nwgpu_graph* g) {
+  if (g->unit) return NWGPU_OK;
+  auto build = [&]() -> int {
+    CK(dalloc(g, &g->unit, g->n), "cudaMalloc(spmv ones)");
+    CK(dalloc(g, &g->zero, g->n), "cudaMalloc(spmv zeros)");
+    spmv_fill_kernel<<<g->sms * 4, 256, 0, g->stream>>>(g->unit, g->n, 1.0f);
+    CK(cudaGetLastError(), "spmv ones");
+    CK(cudaStreamSynchronize(g->stream), "spmv buffers");
+    return NWGPU_OK;
+  };
+  return all_or_none(g, build, [&] {
+    pool_free(g->unit, g->stream);
+    pool_free(g->zero, g->stream);
+    g->unit = g->zero = nullptr;
+  });
+}
 }  // namespace nwgpu
 
 // y = A x over the graph's rows: one sweep of the weighted binned kernel with
@@ -387,13 +421,7 @@ extern "C" int nwgpu_spmv(nwgpu_graph* g, const float* x, float* y, const nwgpu_
   if (n == 0) return NWGPU_OK;
   cudaStream_t s = opt.stream ? (cudaStream_t)opt.stream : g->stream;
   if ((rc = ensure_solve_buffers(g))) return rc;
-  if (!g->unit) {
-    CK(dalloc(g, &g->unit, n), "cudaMalloc(spmv ones)");
-    CK(dalloc(g, &g->zero, n), "cudaMalloc(spmv zeros)");
-    spmv_fill_kernel<<<g->sms * 4, 256, 0, g->stream>>>(g->unit, n, 1.0f);
-    CK(cudaGetLastError(), "spmv ones");
-    CK(cudaStreamSynchronize(g->stream), "spmv buffers");
-  }
+  if ((rc = ensure_spmv(g))) return rc;
   // x in internal order as the sweep's contributions
   const float* xd = x;
   if (!opt.device_ptrs) {

@@ -48,8 +48,17 @@ cudaError_t pool_for_current(cudaMemPool_t* out) {
 }
 }  // namespace
 
+namespace {
+thread_local int64_t t_fail_in = -1;  // allocations of this thread until the one that fails (nwgpu_selftest_fail_allocation)
+
+bool fails_now() { return t_fail_in >= 0 && t_fail_in-- == 0; }
+}  // namespace
+
+void fail_allocation(int64_t after) { t_fail_in = after; }
+
 cudaError_t pool_alloc(void** p, size_t bytes, cudaStream_t s) {
   *p = nullptr;
+  if (fails_now()) return cudaErrorMemoryAllocation;
   cudaMemPool_t pool;
   cudaError_t   e = pool_for_current(&pool);
   if (e != cudaSuccess) return e;
@@ -67,6 +76,7 @@ std::vector<void*> g_host_free;  // cached blocks, each one cudaHostAlloc of kHo
 
 cudaError_t host_block_get(void** p) {
   *p = nullptr;
+  if (fails_now()) return cudaErrorMemoryAllocation;
   {
     std::lock_guard<std::mutex> lock(g_host_mu);
     if (!g_host_free.empty()) {

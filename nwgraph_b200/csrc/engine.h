@@ -175,6 +175,8 @@ cudaError_t pool_alloc_n(T** p, uint64_t count, cudaStream_t s) {
 constexpr size_t kHostBlock = 256;
 cudaError_t host_block_get(void** p);
 void        host_block_put(void* p);
+// The calling thread's pool_alloc / host_block_get call after `after` more fails, once (< 0: none).
+void        fail_allocation(int64_t after);
 
 // graph_build.cu
 cudaError_t validate_csr(const uint32_t* d_row_ptr, const uint32_t* d_col, uint64_t n, uint64_t nnz,

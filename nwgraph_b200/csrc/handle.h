@@ -56,6 +56,7 @@ struct WprBuffers {
   float*     gw = nullptr;       // nnz: dL/dw staging for host outputs
   // GMRES adjoint: Krylov basis (kGmresRestart + 1 vectors of stride ld),
   // operator output, -d/s, per-block reduction partials, reduction results
+  bool       gmres_ready = false;
   float*     basis = nullptr;
   uint64_t   ld = 0;
   float*     w = nullptr;
@@ -66,6 +67,7 @@ struct WprBuffers {
   double*    d_hdots[2] = {nullptr, nullptr};
   float*     f = nullptr;        // n: dL/dw factors d r_j / s_j
   float*     q = nullptr;        // n: dL/dw offsets q_j
+  void       release_gmres(cudaStream_t s);
   void       release(cudaStream_t s);
 };
 
@@ -192,6 +194,18 @@ cudaError_t dalloc(nwgpu_graph* g, T** p, uint64_t count) {
     e = cudaMemsetAsync(*p, 0, bytes, g->stream);
   }
   return e;
+}
+// Runs build() (a status code); if it fails, release() gives back what it got, so the next call starts over and
+// nothing takes a part of the buffers for all of them.
+template <class Build, class Release>
+int all_or_none(nwgpu_graph* g, Build build, Release release) {
+  const uint64_t held = g->device_bytes;
+  const int      rc = build();
+  if (rc) {
+    release();
+    g->device_bytes = held;
+  }
+  return rc;
 }
 int ensure_solve_buffers(nwgpu_graph* g);
 int build_bin_plan(nwgpu_graph* g, const uint32_t* row_ptr, uint64_t n, bool hot, BinPlan* p,
