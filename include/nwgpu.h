@@ -109,6 +109,9 @@ typedef struct nwgpu_graph_info {
   uint32_t chunk_entries;       /* binned: entries per long-row chunk */
   uint32_t bin0_rows_per_warp;  /* binned: rows of 129 entries to the long-row cut-off per warp: 2 (half a warp
                                    each) or 1 (a whole warp); like the cut-offs it sets the rows' summation order */
+  uint32_t kernels_per_sweep;   /* of a plain solve: 2 (the sweep and a finishing kernel), 1 (binned: the sweep's last
+                                   CTA finishes it) or 0 (a small graph: one launch runs the whole solve; decided by
+                                   the handle's first plain or single-seed solve with NWGPU_LAUNCH_GRAPH) */
 } nwgpu_graph_info;
 int nwgpu_graph_get_info(const nwgpu_graph* g, nwgpu_graph_info* info);
 

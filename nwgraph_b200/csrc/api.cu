@@ -1182,7 +1182,13 @@ int nwgpu_graph_get_info(const nwgpu_graph* g, nwgpu_graph_info* info) {
     info->long_row_entries = g->plan.bin.long_row;
     info->chunk_entries = g->plan.bin.chunk;
     info->bin0_rows_per_warp = g->plan.bin.bin0_rows;
+    info->kernels_per_sweep = g->resident.ok ? 0u
+                              : !use_blocked(g, &g->plan, kModePlain) &&
+                                      binned_self_finishing(g->plan.bin, g->plan.hot, kModePlain)
+                                  ? 1u
+                                  : 2u;
   } else {
+    info->kernels_per_sweep = 2u;
     info->sweep_threads = (uint32_t)g->variant.threads;
     info->sweep_grid = (uint32_t)g->grid;
   }

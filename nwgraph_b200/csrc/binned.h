@@ -52,6 +52,8 @@ int         binned_sweep_grid(int sms, bool hot);
 uint32_t    binned_hot_capacity();  // ids the hot variant can stage (a multiple of 4)
 cudaError_t configure_binned_kernels();
 int         binned_finish_grid(const BinnedArgs& a);
+// Whether sweeps of this plan in `mode` are finished by their last CTA (no finishing kernel).
+bool        binned_self_finishing(const BinnedArgs& a, bool hot, int mode);
 // mode: SweepMode. The weighted and adjoint sweeps always use the hot shape
 // (sweep_grid = binned_sweep_grid(sms, true)).
 cudaError_t launch_binned_sweep(const BinnedArgs& a, bool hot, int mode, int sweep_grid, int finish_grid, cudaStream_t s);

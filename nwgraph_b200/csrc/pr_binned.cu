@@ -883,12 +883,16 @@ int binned_finish_grid(const BinnedArgs& a) {
   return blocks ? (int)blocks : 1;
 }
 
+bool binned_self_finishing(const BinnedArgs& a, bool hot, int mode) {
+  return a.fused && binned_fusable(binned_shape_hot(hot, mode), mode);
+}
+
 cudaError_t launch_binned_sweep(const BinnedArgs& a, bool hot, int mode, int sweep_grid, int finish_grid, cudaStream_t s) {
   void*       args[] = {(void*)&a};
   const bool  h = binned_shape_hot(hot, mode);
   cudaError_t e = cudaLaunchKernel(binned_fn(hot, mode), dim3((unsigned)sweep_grid),
                                    dim3(h ? kBinnedHotThreads : kBinnedThreads), args, h ? (size_t)a.smem_ids * 4u : 0u, s);
-  if (e != cudaSuccess || (a.fused && binned_fusable(h, mode))) return e;
+  if (e != cudaSuccess || binned_self_finishing(a, hot, mode)) return e;
   return cudaLaunchKernel(binned_finish_fn(mode), dim3((unsigned)finish_grid), dim3(256), args, 0, s);
 }
 
@@ -905,7 +909,7 @@ cudaError_t add_binned_nodes(cudaGraph_t body, const BinnedArgs& a, bool hot, in
   cudaGraphNode_t sn, fn;
   cudaError_t     e = cudaGraphAddKernelNode(&sn, body, nullptr, 0, &kp);
   if (e != cudaSuccess) return e;
-  if (a.fused && binned_fusable(h, mode)) {
+  if (binned_self_finishing(a, hot, mode)) {
     // more sweeps per round of the while loop, whose own step costs about 5 us, a kernel after a kernel 2: a sweep
     // after the last one returns at once (a personalised solve of 14 sweeps at RMAT scale 20: 1439 to 1386 us)
     for (int i = 1; i < kLoopSweeps; ++i) {
