@@ -416,6 +416,19 @@ void ResidentPlan::release(cudaStream_t s) {
 // sixteen of them one (both from the L2 paths' rates), and the share of
 // gathers that hit the first H ids is the share of entries in their rows
 // (exact where the graph is symmetric).
+//
+// A sweep of the resident kernel takes as long as its fullest CTA's gathers
+// past the hubs, in 32-byte sectors; the sweep loop spreads them over all SMs
+// and has more room for hubs. So the first is the faster one up to a number of
+// them. 20 sweeps, loop against resident, by the fullest CTA's sectors:
+// without long rows (uniform and mildly skewed random graphs, bands, grids)
+// 1.2 and more up to 10,000, 1.05 to 1.17 at 11,000 to 13,000, 0.97 to 1.16 at
+// 13,600 to 17,200, 0.80 to 0.94 at 20,000 to 25,000, 0.7 at 32,000. With
+// long rows (RMAT), for whose chunks the loop waits, 1.1 to 1.3 at 17,000 to
+// 26,500 sectors of 20,000 to 32,000 gathers, 0.70 to 0.88 from 50,000
+// gathers on, where no room is left for hubs (none lies between) -- unless one
+// CTA has most of the work: 0.73 with 34,000 entries beside an average of
+// 2300, 0.92 with 30,000 beside 8300, but 1.19 beside 15,000.
 static int ensure_resident(nwgpu_graph* g) {
   ResidentPlan& p = g->resident;
   if (p.tried) return NWGPU_OK;
@@ -436,10 +449,11 @@ static int ensure_resident(nwgpu_graph* g) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
   pool_free(d, g->stream);
   CK(e, "resident bounds");
-  uint64_t most = 0, most_entries = 0;
+  uint64_t most = 0, most_entries = 0, fullest = 0;  // fullest: that CTA's first entry
   for (int c = 0; c < C; ++c) {
     const uint64_t E = h[C + 2 + c] - h[C + 1 + c], R = h[c + 1] - h[c];
     most = std::max(most, resident_words(E, R));
+    if (E > most_entries) fullest = h[C + 1 + c];
     most_entries = std::max(most_entries, E);
   }
   const uint64_t limit = resident_smem_limit() / 4u;
@@ -452,6 +466,18 @@ static int ensure_resident(nwgpu_graph* g) {
       best = cost;
       p.hub_ids = (uint32_t)H;
     }
+  }
+  if (most_entries > kResidentSectors) {
+    uint32_t counts[2] = {0, 0};  // gathers, sectors
+    if ((e = pool_alloc_n(&d, 2, g->stream)) == cudaSuccess) e = cudaMemsetAsync(d, 0, sizeof(counts), g->stream);
+    if (e == cudaSuccess) e = launch_resident_gathers(g->g.col + fullest, (uint32_t)most_entries, p.hub_ids, d, g->stream);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(counts, d, sizeof(counts), cudaMemcpyDeviceToHost, g->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(g->stream);
+    pool_free(d, g->stream);
+    CK(e, "resident gathers");
+    const bool even_skew =
+        g->plan.bin.num_long_rows && (double)most_entries <= kResidentUneven * (double)g->nnz / (double)C;
+    if (counts[1] > kResidentSectors && !(even_skew && counts[0] <= kResidentSkewedGathers)) return NWGPU_OK;
   }
   p.smem_bytes = (uint32_t)(most + p.hub_ids) * 4u;
   p.ctas = C;

@@ -362,6 +362,36 @@ __global__ void resident_bounds_kernel(const uint32_t* __restrict__ row_ptr, uin
   }
 }
 
+// A thread per entry; the sectors' numbers go into a hash set (at most 1024 of them in 4096 places, so every probe ends).
+__global__ void __launch_bounds__(1024) resident_gathers_kernel(const uint32_t* __restrict__ col, uint32_t entries,
+                                                                uint32_t hub_ids, uint32_t* __restrict__ counts) {
+  constexpr uint32_t  kPlaces = 4096, kNone = 0xffffffffu;
+  __shared__ uint32_t s_set[kPlaces];
+  for (uint32_t i = threadIdx.x; i < kPlaces; i += 1024u) s_set[i] = kNone;
+  __syncthreads();
+  const uint32_t e = blockIdx.x * 1024u + threadIdx.x, id = e < entries ? col[e] : 0u;
+  const bool     past = e < entries && id >= hub_ids;
+  bool           is_new = false;
+  if (past) {
+    const uint32_t sector = id >> 3;
+    for (uint32_t at = (sector * 2654435761u) >> 20;; at = (at + 1u) % kPlaces) {
+      const uint32_t was = atomicCAS(s_set + at, kNone, sector);
+      is_new = was == kNone;
+      if (is_new || was == sector) break;
+    }
+  }
+  const int gathers = __syncthreads_count(past), sectors = __syncthreads_count(is_new);
+  if (threadIdx.x == 0) {
+    atomicAdd(counts, (uint32_t)gathers);
+    atomicAdd(counts + 1, (uint32_t)sectors);
+  }
+}
+
+cudaError_t launch_resident_gathers(const uint32_t* col, uint32_t entries, uint32_t hub_ids, uint32_t* counts, cudaStream_t s) {
+  resident_gathers_kernel<<<(entries + 1023u) / 1024u, 1024, 0, s>>>(col, entries, hub_ids, counts);
+  return cudaGetLastError();
+}
+
 cudaError_t launch_resident_bounds(const uint32_t* row_ptr, uint64_t n, uint64_t nnz, int ctas, uint32_t* bounds,
                                    uint32_t* out, cudaStream_t s) {
   const unsigned threads = (unsigned)ctas + 1u + kNumResidentHubs;

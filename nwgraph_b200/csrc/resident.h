@@ -56,6 +56,11 @@ constexpr unsigned int kFaultResidentWait = 0x52455349u;  // PrState::fault: a g
 
 // Largest entry count the resident solve is considered for.
 constexpr uint64_t kResidentMaxEntries = 8ull << 20;
+// What the fullest CTA may gather past the hubs per sweep (ensure_resident has the measurements): of any graph, in
+// sectors; of one with long rows and no CTA above kResidentUneven times the average, in gathers.
+constexpr uint32_t kResidentSectors = 17000;
+constexpr uint32_t kResidentSkewedGathers = 33000;
+constexpr double   kResidentUneven = 2.5;
 
 cudaError_t configure_resident_kernel();
 // Row bounds of `ctas` ranges of about equal work into bounds[0..ctas]; what the host sizes the plan by into
@@ -63,6 +68,9 @@ cudaError_t configure_resident_kernel();
 constexpr uint32_t kNumResidentHubs = 8, kResidentHubStep = 6144;
 cudaError_t launch_resident_bounds(const uint32_t* row_ptr, uint64_t n, uint64_t nnz, int ctas, uint32_t* bounds,
                                    uint32_t* out, cudaStream_t s);
+// counts[0], counts[1] (zeroed) += among the `entries` entries at col, the gathers past the first hub_ids
+// contributions and, per 1024 consecutive entries, the distinct 32-byte sectors they fall in.
+cudaError_t launch_resident_gathers(const uint32_t* col, uint32_t entries, uint32_t hub_ids, uint32_t* counts, cudaStream_t s);
 int      resident_ctas(uint64_t n, uint64_t nnz, int sms);
 uint64_t resident_words(uint64_t E, uint64_t R);
 uint32_t resident_smem_limit();

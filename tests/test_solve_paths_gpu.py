@@ -22,8 +22,9 @@ def _kernels(rp, col, relabel=True, launch="graph"):
 
 @pytest.mark.parametrize("kind", KINDS)
 def test_the_resident_tests_graphs_are_resident(gpu, kind):
-    # (one vertex is not relabelled: the merge-path sweep)
-    assert _kernels(*_graph(kind)) == (2 if kind == "one vertex" else 0)
+    # (one vertex is not relabelled: the merge-path sweep; "warp of chunks" has four rows of 16 times a CTA's share,
+    # which the loop solves faster: test_rows_of_many_chunks_in_one_launch has its chunks)
+    assert _kernels(*_graph(kind)) == {"one vertex": 2, "warp of chunks": 1}.get(kind, 0)
 
 
 def test_the_other_paths(gpu, monkeypatch):
@@ -36,3 +37,61 @@ def test_the_other_paths(gpu, monkeypatch):
     assert _kernels(g.row_ptr, g.col) == 1
     monkeypatch.setenv("NWGPU_SWEEP", "binned")  # the 256-thread shape
     assert _kernels(g.row_ptr, g.col) == 2
+
+
+def _even_rows(n, per_row, band):
+    """Rows of equal length; neighbours anywhere (band 0) or at most `band` ids on."""
+    rng = np.random.default_rng(7)
+    rp = (np.arange(n + 1, dtype=np.int64) * per_row).astype(np.uint32)
+    if band:
+        col = (np.repeat(np.arange(n), per_row) + rng.integers(1, band + 1, n * per_row)) % n
+    else:
+        col = rng.integers(0, n, n * per_row)
+    return rp, col.astype(np.uint32)
+
+
+def _hubs(lens, n, rest):
+    rng = np.random.default_rng(8)
+    rp = np.zeros(n + 1, np.uint32)
+    rp[1:] = np.cumsum(np.concatenate([lens, np.full(n - len(lens), rest)]))
+    return rp, rng.integers(0, n, int(rp[-1])).astype(np.uint32)
+
+
+@pytest.mark.parametrize("make,kernels", [
+    (lambda: _even_rows(1 << 17, 12, 0), 0),         # 10,600 entries a CTA, few past the hubs
+    (lambda: _even_rows(1 << 17, 32, 0), 1),         # 28,300, three quarters past them: the loop is 1.1 times as fast
+    (lambda: _even_rows(600000, 6, 0), 1),           # 24,300, nearly all past them: 1.2 times
+    (lambda: _even_rows(1 << 18, 14, 30), 0),        # 24,800, but neighbours share sectors
+    (lambda: _hubs([34000] * 4, 70000, 3), 1),       # one CTA has fourteen times the average: 1.4 times
+    (lambda: _hubs([14000] * 4, 70000, 3), 0),       # six times, but few
+])
+def test_graphs_the_sweep_loop_solves_faster_keep_it(gpu, make, kernels):
+    rp, col = make()
+    n = len(rp) - 1
+    deg = np.bincount(col, minlength=n).astype(np.uint32)
+    a, b = np.empty(n, np.float32), np.empty(n, np.float32)
+    with Graph(rp, col) as g:
+        sa = g.page_rank(deg, a, 0.85, 1e-6, 20)
+        assert g.info()["kernels_per_sweep"] == kernels
+        sb = g.page_rank(deg, b, 0.85, 1e-6, 20, launch="stream")
+    assert np.array_equal(a, b, equal_nan=True) and sa.iterations == sb.iterations
+
+
+def test_rows_of_many_chunks_in_one_launch(gpu, monkeypatch):
+    """Rows of 32 and more chunks, which the last case above but one leaves to the loop at the default cut-offs."""
+    rp, col = _hubs([8191, 8192, 8193, 12000, 16385], 70000, 3)
+    n = len(rp) - 1
+    deg = np.bincount(col, minlength=n).astype(np.uint32)
+    a, b = np.empty(n, np.float32), np.empty(n, np.float32)
+    monkeypatch.setenv("NWGPU_CHUNK_ENTRIES", "256")
+    with Graph(rp, col) as g:
+        sa = g.page_rank(deg, a, 0.85, 1e-6, 20)
+        assert g.info()["kernels_per_sweep"] == 0
+        sb = g.page_rank(deg, b, 0.85, 1e-6, 20, launch="stream")
+    assert np.array_equal(a, b, equal_nan=True) and sa.iterations == sb.iterations
+
+
+@pytest.mark.parametrize("edge_factor,kernels", [(20, 0), (28, 1)])  # hubs beside the rows, or no room for them
+def test_hubs_without_room(gpu, edge_factor, kernels):
+    g = G.rmat(17, edge_factor, 5)
+    assert _kernels(g.row_ptr, g.col) == kernels
