@@ -190,6 +190,8 @@ typedef struct nwgpu_ppr_stats {
  * order (column c = the vector of seeds[c]). Each column stops at its own
  * first sweep whose FP64 L1 change is < threshold (its values then stay
  * fixed) or at max_iters. One column-index load feeds all k gathers.
+ * The handle keeps the n x k work matrices of its widest batch (this call's
+ * and the two below); narrower batches use a part of them.
  * No counterpart in the reference. */
 int nwgpu_ppr_batched(nwgpu_graph* g, const uint32_t* out_degree, const uint32_t* seeds, uint32_t k, float* ranks_nxk,
                       float damping, float threshold, uint64_t max_iters, const nwgpu_pr_options* options,

@@ -8,13 +8,26 @@
 
 namespace nwgpu {
 
-void PprBuffers::release(cudaStream_t s) {
-  if (cg_exec) cudaGraphExecDestroy(cg_exec);
+void PprLoop::release() {
+  if (exec) cudaGraphExecDestroy(exec);
   if (cg) cudaGraphDestroy(cg);
-  cg_exec = nullptr;
-  cg = nullptr;
-  void* ptrs[] = {tiling.tile_row, tiling.tile_nnz, rank, contrib[0], contrib[1], out, cpart, epart, res_part,
-                  end_bits, full_rows, tile_full, spans, seeds, seeds_in, col_done, col_conv, col_iters, col_err, st, vbase, slot_map, slot_orig};
+  *this = PprLoop();
+}
+
+void PprBuffers::release_matrices(cudaStream_t s) {
+  for (PprLoop& l : loops) l.release();
+  void* ptrs[] = {rank, contrib[0], contrib[1], out, cpart, epart, res_part, vbase};
+  for (void* p : ptrs) pool_free(p, s);
+  rank = contrib[0] = contrib[1] = out = cpart = epart = vbase = nullptr;
+  res_part = nullptr;
+  K = 0;
+  matrix_bytes = 0;
+}
+
+void PprBuffers::release(cudaStream_t s) {
+  release_matrices(s);
+  void* ptrs[] = {tiling.tile_row, tiling.tile_nnz, end_bits, full_rows, tile_full, spans, seeds, seeds_in,
+                  col_done, col_conv, col_iters, col_err, slot_map, slot_orig, st};
   for (void* p : ptrs) pool_free(p, s);
   if (h_st) {
     cudaStreamSynchronize(s);  // no copy may still target the block when it is reused
@@ -47,29 +60,23 @@ static int list_full_rows(nwgpu_graph* g, uint32_t* rows) {
   return NWGPU_OK;
 }
 
-static int build_ppr(nwgpu_graph* g, int K) {
+// What does not depend on the batch's width: tiles, rows crossing them, the
+// rows' last entries, the columns' words.
+static int build_ppr(nwgpu_graph* g) {
   PprBuffers&    b = g->ppr;
-  const uint64_t n = g->n, nk = g->n * (uint64_t)K;
+  const uint64_t n = g->n;
   CK(build_tiling(g->g.row_ptr, n, g->nnz, (uint32_t)kPprTileItems, &b.tiling, g->stream), "ppr tiling");
   const uint64_t T = b.tiling.num_tiles;
   b.finish_grid = g->sms * 4;
-  CK(dalloc(g, &b.rank, nk), "cudaMalloc(ppr rank)");
-  CK(dalloc(g, &b.contrib[0], nk), "cudaMalloc(ppr contrib)");
-  CK(dalloc(g, &b.contrib[1], nk), "cudaMalloc(ppr contrib)");
-  CK(dalloc(g, &b.out, nk), "cudaMalloc(ppr out)");
-  CK(dalloc(g, &b.cpart, (T + 1) * K), "cudaMalloc(ppr cpart)");
-  CK(dalloc(g, &b.epart, (T + 1) * K), "cudaMalloc(ppr epart)");
-  CK(dalloc(g, &b.res_part, (uint64_t)b.finish_grid * K), "cudaMalloc(ppr res)");
-  CK(dalloc(g, &b.seeds, (uint64_t)K), "cudaMalloc(seeds)");
-  CK(dalloc(g, &b.seeds_in, (uint64_t)K), "cudaMalloc(seeds)");
-  CK(dalloc(g, &b.col_done, (uint64_t)K), "cudaMalloc(col flags)");
-  CK(dalloc(g, &b.col_conv, (uint64_t)K), "cudaMalloc(col flags)");
-  CK(dalloc(g, &b.col_iters, (uint64_t)K), "cudaMalloc(col iters)");
-  CK(dalloc(g, &b.col_err, (uint64_t)K), "cudaMalloc(col err)");
+  CK(dalloc(g, &b.seeds, kPprMaxK), "cudaMalloc(seeds)");
+  CK(dalloc(g, &b.seeds_in, kPprMaxK), "cudaMalloc(seeds)");
+  CK(dalloc(g, &b.col_done, kPprMaxK), "cudaMalloc(col flags)");
+  CK(dalloc(g, &b.col_conv, kPprMaxK), "cudaMalloc(col flags)");
+  CK(dalloc(g, &b.col_iters, kPprMaxK), "cudaMalloc(col iters)");
+  CK(dalloc(g, &b.col_err, kPprMaxK), "cudaMalloc(col err)");
   CK(dalloc(g, &b.st, 1), "cudaMalloc(ppr state)");
-  CK(dalloc(g, &b.slot_map, (uint64_t)K), "cudaMalloc(ppr slots)");
-  CK(dalloc(g, &b.slot_orig, (uint64_t)K), "cudaMalloc(ppr slots)");
-  // rows crossing tiles and the rows' last entries, once per graph
+  CK(dalloc(g, &b.slot_map, kPprMaxK), "cudaMalloc(ppr slots)");
+  CK(dalloc(g, &b.slot_orig, kPprMaxK), "cudaMalloc(ppr slots)");
   CK(dalloc(g, &b.spans, T + 1), "cudaMalloc(ppr spans)");
   CK(dalloc(g, &b.end_bits, g->nnz / 32 + 1), "cudaMalloc(ppr row ends)");
   {
@@ -98,14 +105,46 @@ static int build_ppr(nwgpu_graph* g, int K) {
   static_assert(sizeof(PprState) <= kHostBlock, "state mirror fits a host block");
   CK(host_block_get((void**)&b.h_st), "cudaHostAlloc(ppr state)");
   CK(cudaStreamSynchronize(g->stream), "ppr buffers");
+  b.ready = true;
+  return NWGPU_OK;
+}
+
+static int build_ppr_matrices(nwgpu_graph* g, int K) {
+  PprBuffers&    b = g->ppr;
+  const uint64_t n = g->n, nk = n * (uint64_t)K, T = b.tiling.num_tiles, held = g->device_bytes;
+  CK(dalloc(g, &b.rank, nk), "cudaMalloc(ppr rank)");
+  CK(dalloc(g, &b.contrib[0], nk), "cudaMalloc(ppr contrib)");
+  CK(dalloc(g, &b.contrib[1], nk), "cudaMalloc(ppr contrib)");
+  CK(dalloc(g, &b.out, nk), "cudaMalloc(ppr out)");
+  CK(dalloc(g, &b.cpart, (T + 1) * K), "cudaMalloc(ppr cpart)");
+  CK(dalloc(g, &b.epart, (T + 1) * K), "cudaMalloc(ppr epart)");
+  CK(dalloc(g, &b.res_part, (uint64_t)b.finish_grid * K), "cudaMalloc(ppr res)");
+  CK(cudaStreamSynchronize(g->stream), "ppr buffers");
+  b.matrix_bytes = g->device_bytes - held;
   b.K = K;
   return NWGPU_OK;
 }
 
-static int ensure_ppr(nwgpu_graph* g, int K) {
-  if (g->ppr.K == K) return NWGPU_OK;
-  g->ppr.release(g->stream);
-  return all_or_none(g, [&] { return build_ppr(g, K); }, [&] { g->ppr.release(g->stream); });
+// A handle keeps the matrices of its widest batch, and a loop graph per width:
+// one that answers batches of 6, 12 and 20 seeds in turn allocates, clears and
+// builds nothing after the first round (RMAT scale 18: 2.51 to 2.08 ms a call
+// against making all of it anew whenever the width changes).
+static int ensure_ppr(nwgpu_graph* g, int K, bool base_terms) {
+  PprBuffers& b = g->ppr;
+  int         rc = NWGPU_OK;
+  if (!b.ready && (rc = all_or_none(g, [&] { return build_ppr(g); }, [&] { b.release(g->stream); }))) return rc;
+  if (b.K < K) {
+    g->device_bytes -= b.matrix_bytes;
+    b.release_matrices(g->stream);
+    if ((rc = all_or_none(g, [&] { return build_ppr_matrices(g, K); }, [&] { b.release_matrices(g->stream); }))) return rc;
+  }
+  if (base_terms && !b.vbase) {
+    const uint64_t held = g->device_bytes;
+    CK(dalloc(g, &b.vbase, g->n * (uint64_t)b.K), "cudaMalloc(ppr base terms)");
+    CK(cudaStreamSynchronize(g->stream), "ppr buffers");
+    b.matrix_bytes += g->device_bytes - held;
+  }
+  return NWGPU_OK;
 }
 
 int ppr_loop(nwgpu_graph* g, const PprArgs& a, int K, uint32_t k, float* ranks_nxk, float damping, uint64_t max_iters,
@@ -116,7 +155,7 @@ static int padded_k(const nwgpu_graph* g, uint32_t k, int mode) {
   return ppr_padded_k(k, mode, ppr_few_tiles((items + kPprTileItems - 1) / kPprTileItems, g->sms));
 }
 
-static PprArgs make_ppr_args(nwgpu_graph* g, float damping) {
+static PprArgs make_ppr_args(nwgpu_graph* g, int K, float damping) {
   PprBuffers& b = g->ppr;
   PprArgs     a = {};
   a.row_ptr = g->g.row_ptr;
@@ -135,7 +174,7 @@ static PprArgs make_ppr_args(nwgpu_graph* g, float damping) {
   a.res_part = b.res_part;
   a.epi_grid = (uint32_t)b.finish_grid;
   a.n = g->n;
-  a.K = (uint32_t)b.K;
+  a.K = (uint32_t)K;
   a.end_bits = b.end_bits;
   a.num_full = b.num_full;
   a.full_rows = b.full_rows;
@@ -192,12 +231,12 @@ extern "C" int nwgpu_ppr_batched(nwgpu_graph* g, const uint32_t* out_degree, con
   }
   int rc = ensure_solve_buffers(g);
   if (rc) return rc;
-  if ((rc = ensure_ppr(g, K))) return rc;
+  if ((rc = ensure_ppr(g, K, false))) return rc;
   PprBuffers&  b = g->ppr;
   cudaStream_t s = opt.stream ? (cudaStream_t)opt.stream : g->stream;
   *(volatile unsigned int*)g->h_abort = 0u;
   if ((rc = load_degrees(g, out_degree, opt.device_ptrs != 0, s))) return rc;
-  PprArgs a = make_ppr_args(g, damping);
+  PprArgs a = make_ppr_args(g, K, damping);
   CK(cudaMemcpyAsync(b.seeds_in, h_seeds, k * sizeof(uint32_t), cudaMemcpyHostToDevice, s), "copy seeds");
   CK(launch_ppr_seeds(b.seeds_in, k, K, g->relabelled ? g->g.perm : nullptr, a, s), "ppr seeds");
   PprState h = {};
@@ -260,19 +299,20 @@ int ppr_loop(nwgpu_graph* g, const PprArgs& a0, int K0, uint32_t k, float* ranks
   };
   CK(cudaEventRecord(g->ev0, s), "cudaEventRecord");
   if (opt.launch == NWGPU_LAUNCH_GRAPH) {
-    if (!b.cg_exec || b.cg_damping != damping || b.cg_mode != mode) {
-      if (b.cg_exec) cudaGraphExecDestroy(b.cg_exec);
-      if (b.cg) cudaGraphDestroy(b.cg);
-      b.cg_exec = nullptr;
-      CK(cudaGraphCreate(&b.cg, 0), "cudaGraphCreate");
-      CK(build_ppr_graph(b.cg, a, K, ppr_sweep_grid(K, mode, few_tiles, g->sms), b.st, &b.cg_exec), "ppr graph");
-      b.cg_damping = damping;
-      b.cg_mode = mode;
+    int width = 0;
+    while ((kPprMinK << width) < K) ++width;
+    PprLoop& loop = b.loops[width];
+    if (!loop.exec || loop.damping != damping || loop.mode != mode) {
+      loop.release();
+      CK(cudaGraphCreate(&loop.cg, 0), "cudaGraphCreate");
+      CK(build_ppr_graph(loop.cg, a, K, ppr_sweep_grid(K, mode, few_tiles, g->sms), b.st, &loop.exec), "ppr graph");
+      loop.damping = damping;
+      loop.mode = mode;
     }
     const uint64_t max_launches = max_iters / kGraphChunk + 2;
     for (uint64_t l = 0;; ++l) {
       if (l == max_launches) return fail(NWGPU_ERR_CUDA, "ppr sweep loop did not finish");
-      CK(cudaGraphLaunch(b.cg_exec, s), "cudaGraphLaunch");
+      CK(cudaGraphLaunch(loop.exec, s), "cudaGraphLaunch");
       CK(cudaMemcpyAsync(b.h_st, b.st, sizeof(PprState), cudaMemcpyDeviceToHost, s), "copy ppr state");
       CK(cudaStreamSynchronize(s), "ppr sweep loop");
       if (b.h_st->done) break;
@@ -411,9 +451,8 @@ static int teleport_batched(nwgpu_graph* g, bool weighted, const uint32_t* out_d
   int rc = ensure_solve_buffers(g);
   if (rc) return rc;
   if (weighted && (rc = ensure_wpr(g))) return rc;  // out-weight sums (internal order)
-  if ((rc = ensure_ppr(g, K))) return rc;
-  PprBuffers& b = g->ppr;
-  if (!b.vbase) CK(dalloc(g, &b.vbase, n * (uint64_t)K), "cudaMalloc(ppr base terms)");
+  if ((rc = ensure_ppr(g, K, true))) return rc;
+  PprBuffers&  b = g->ppr;
   cudaStream_t s = opt.stream ? (cudaStream_t)opt.stream : g->stream;
   *(volatile unsigned int*)g->h_abort = 0u;
   if (!weighted && (rc = load_degrees(g, out_degree, opt.device_ptrs != 0, s))) return rc;
@@ -423,7 +462,7 @@ static int teleport_batched(nwgpu_graph* g, bool weighted, const uint32_t* out_d
     CK(cudaMemcpyAsync(b.out, teleports, n * k * sizeof(float), cudaMemcpyHostToDevice, s), "copy teleports");
     t = b.out;
   }
-  PprArgs a = make_ppr_args(g, damping);
+  PprArgs a = make_ppr_args(g, K, damping);
   a.vbase = b.vbase;
   if (weighted) {
     a.w = g->g.w;

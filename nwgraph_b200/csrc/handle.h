@@ -71,38 +71,50 @@ struct WprBuffers {
   void       release(cudaStream_t s);
 };
 
-// Buffers of the batched personalised solve (K padded columns).
+// CUDA graph of the batched solve's sweep loop at one width.
+struct PprLoop {
+  cudaGraph_t     cg = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  float           damping = -1.f;
+  int             mode = -1;  // ppr_mode of the solve baked into exec
+  void            release();
+};
+
+// Buffers of the batched personalised solve.
 struct PprBuffers {
-  int             K = 0;
+  // What the graph's rows fix, at any width (made by the first batch).
+  bool            ready = false;
   Tiling          tiling{};  // tiles of kPprTileItems
   int             finish_grid = 0;  // epilogue CTAs
-  float*          rank = nullptr;
-  float*          contrib[2] = {nullptr, nullptr};
-  float*          out = nullptr;  // n x K staging for the output
-  float*          cpart = nullptr;
-  float*          epart = nullptr;
-  double*         res_part = nullptr;
   uint32_t*       end_bits = nullptr;   // one bit per entry: the last of its row
   uint32_t*       full_rows = nullptr;  // rows that have entries, where others lie between them
   uint32_t*       tile_full = nullptr;  // per tile: its first row's place in full_rows
   uint32_t        num_full = 0;
   uint4*          spans = nullptr;  // rows crossing tiles
   uint32_t        num_spans = 0;
+  // One word per column, kPprMaxK of each.
   uint32_t*       seeds = nullptr;
   uint32_t*       seeds_in = nullptr;
   uint32_t*       col_done = nullptr;
   uint32_t*       col_conv = nullptr;
   uint32_t*       col_iters = nullptr;
   double*         col_err = nullptr;
-  PprState*       st = nullptr;
-  PprState*       h_st = nullptr;
-  cudaGraph_t     cg = nullptr;
-  cudaGraphExec_t cg_exec = nullptr;
-  float           cg_damping = -1.f;
-  int             cg_mode = -1;  // ppr_mode of the solve baked into cg_exec
-  float*          vbase = nullptr;  // weighted solves: n x K base terms (1 - d) t
   uint32_t*       slot_map = nullptr;   // narrowing: old slot of each new slot
   uint32_t*       slot_orig = nullptr;  // caller's column held by each slot (>= k: none)
+  PprState*       st = nullptr;
+  PprState*       h_st = nullptr;
+  // Matrices of K columns, those of the widest batch so far; a narrower one uses the front of each.
+  int             K = 0;
+  uint64_t        matrix_bytes = 0;  // device memory of the matrices
+  float*          rank = nullptr;
+  float*          contrib[2] = {nullptr, nullptr};
+  float*          out = nullptr;  // n x K staging for the output
+  float*          cpart = nullptr;
+  float*          epart = nullptr;
+  double*         res_part = nullptr;
+  float*          vbase = nullptr;  // teleport matrices: n x K base terms (1 - d) t
+  PprLoop         loops[kPprWidths];  // of kPprMinK << i columns, over these matrices
+  void            release_matrices(cudaStream_t s);
   void            release(cudaStream_t s);  // returns the buffers to the pool on stream s
 };
 

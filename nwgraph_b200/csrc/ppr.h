@@ -8,6 +8,7 @@ namespace nwgpu {
 
 constexpr int kPprTileItems = 512;  // merge items per tile
 constexpr int kPprThreads = 256;    // gather CTA
+constexpr int kPprMinK = 8, kPprMaxK = 128, kPprWidths = 5;  // padded widths: 8, 16, 32, 64, 128
 // Sweeps per round of the device-side loop, whose own step costs about 5 us; sweeps after the last return at once.
 constexpr int kPprLoopSweeps = 3;
 // What a batched solve's columns are: one-hot teleports at seeds; teleport
