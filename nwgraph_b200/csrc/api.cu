@@ -338,7 +338,7 @@ int build_bin_plan(nwgpu_graph* g, const uint32_t* row_ptr, uint64_t n64, bool h
     if (e != cudaSuccess) return cuda_fail(e, "chunk table");
   }
   b.num_chunks = num_chunks;
-  b.fused = num_chunks <= kFuseChunks ? 1u : 0u;
+  b.fused = (uint64_t)num_chunks + (uint64_t)kFuseRow * nlong <= kFuseWork ? 1u : 0u;
   CK(dalloc(g, &p->chunk_row, (uint64_t)num_chunks), "cudaMalloc(chunk rows)");
   CK(dalloc(g, &p->chunk_part, (uint64_t)num_chunks), "cudaMalloc(chunk partials)");
   CK(launch_chunk_fill(p->first, nlong, p->chunk_row, g->sms, g->stream), "chunk fill");

@@ -11,8 +11,16 @@ constexpr uint32_t kChunk = 1024;    // entries per long-row chunk (one warp)
 constexpr uint32_t kBin0Rows = 2;    // bin-0 rows per warp: 2 (half a warp each) or 1 (a whole warp)
 constexpr int      kNumBins = 8;     // warp per row, then G = 32, 16, 8, 4, 2, 1, empty
 
-// Plans of at most this many chunks are finished by the sweep's last CTA.
-constexpr uint32_t kFuseChunks = 32768;
+// Plans of at most this much finishing work -- partials to add, a long row's
+// own bounds, inputs and update counting as five -- are finished by the
+// sweep's last CTA; others by a kernel on all SMs. Per sweep of a solve, with
+// the kernel against without it (us): 1351 long rows in 7263 chunks (work
+// 14,000) 100.7 to 97.2, 2051 in 14,001 (24,300) 190.6 to 188.1, 4096 in 12,288
+// (32,800) 70.6 to 69.0, 5500 in 16,500 (44,000) 78.2 to 76.8, 4096 in 28,672 and
+// 6144 in 18,432 (49,200 both) 135.4 to 136.6 and 81.3 to 81.0, 6194 in 26,659
+// (57,600) 150.6 to 152.9, 10,900 in 32,700 (87,200) 116.2 to 118.6.
+constexpr uint32_t kFuseWork = 48000;
+constexpr uint32_t kFuseRow = 5;
 constexpr int      kLoopSweeps = 3;  // of such a plan, per round of the device-side loop
 
 struct BinnedArgs {
@@ -23,7 +31,7 @@ struct BinnedArgs {
   uint32_t        num_long_rows;          // rows [0, num_long_rows) are chunked
   uint32_t        num_big_rows;           // rows [0, num_big_rows) have more than 32 chunks
   uint32_t        num_chunks;
-  uint32_t        fused;                  // the sweep's last CTA finishes the long rows and the sweep (kFuseChunks)
+  uint32_t        fused;                  // the sweep's last CTA finishes the long rows and the sweep (kFuseWork)
   const uint32_t* row_first_chunk;        // num_long_rows + 1
   const uint32_t* chunk_row;              // num_chunks
   float*          chunk_part;             // num_chunks partial sums

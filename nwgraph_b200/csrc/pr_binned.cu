@@ -24,7 +24,7 @@
 //
 // The long rows are finished after the sweep, and the FP64 residual partials
 // reduced in a fixed order for the convergence test on the device: by the
-// sweep's last CTA to end (a ticket) where the chunks are few, else by
+// sweep's last CTA to end (a ticket) where they are little work, else by
 // pr_binned_finish_kernel, launched right after. A kernel of its own cost 10 us
 // at RMAT scale 20 (its launch, row bounds, partials and rows one after
 // another) and the last CTA does it in about 4, with one fence per CTA; at scale
@@ -579,7 +579,7 @@ __host__ __device__ constexpr bool binned_fusable(bool hot, int mode) { return h
 // ---------------------------------------------------------------------------
 // Finishing: the long rows' sums from their chunk partials, then the residual
 // and the convergence test. The last CTA of the sweep to finish does it where
-// the chunks are few (BinnedArgs::fused); else a kernel of its own, which has
+// that is little work (BinnedArgs::fused); else a kernel of its own, which has
 // all SMs for them.
 // ---------------------------------------------------------------------------
 // Virtual thread gt of the long rows: rows [0, num_big_rows) have more than 32

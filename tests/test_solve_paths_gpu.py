@@ -95,3 +95,30 @@ def test_rows_of_many_chunks_in_one_launch(gpu, monkeypatch):
 def test_hubs_without_room(gpu, edge_factor, kernels):
     g = G.rmat(17, edge_factor, 5)
     assert _kernels(g.row_ptr, g.col) == kernels
+
+
+@pytest.mark.parametrize("rows,per_row,kernels", [
+    (5333, 4000, 1),   # 21,332 chunks: 47,997
+    (5334, 4000, 2),
+    (1000, 44000, 1),  # rows of 43 chunks: 48,000
+    (1001, 44000, 2),
+])
+def test_finishing_work(gpu, monkeypatch, rows, per_row, kernels):
+    """Both sides of the line between the last CTA and a kernel for the long rows: chunks + 5 rows, against 48,000. The
+    ranks depend on neither."""
+    rp, col = _hubs([per_row] * rows, 60000, 2)
+    chunks = rows * -(-per_row // 1024)
+    assert (chunks + 5 * rows <= 48000) == (kernels == 1)
+    n = len(rp) - 1
+    deg = np.bincount(col, minlength=n).astype(np.uint32)
+    a, b = np.empty(n, np.float32), np.empty(n, np.float32)
+    with Graph(rp, col) as g:
+        sa = g.page_rank(deg, a, 0.85, 0.0, 7, record_errors=True)
+        assert g.info()["kernels_per_sweep"] == kernels
+        for launch in ("graph", "stream"):
+            sb = g.page_rank(deg, b, 0.85, 0.0, 7, launch=launch, record_errors=True)
+            assert np.array_equal(a, b) and np.array_equal(sa.errors, sb.errors)
+    monkeypatch.setenv("NWGPU_SWEEP", "binned")  # the 256-thread shape has a finishing kernel always
+    with Graph(rp, col) as g:
+        g.page_rank(deg, b, 0.85, 0.0, 7)
+    assert np.array_equal(a, b)
