@@ -338,7 +338,7 @@ int build_bin_plan(nwgpu_graph* g, const uint32_t* row_ptr, uint64_t n64, bool h
     if (e != cudaSuccess) return cuda_fail(e, "chunk table");
   }
   b.num_chunks = num_chunks;
-  b.fused = (uint64_t)num_chunks + (uint64_t)kFuseRow * nlong <= kFuseWork ? 1u : 0u;
+  b.fused = !g->finish_apart && (uint64_t)num_chunks + (uint64_t)kFuseRow * nlong <= kFuseWork ? 1u : 0u;
   CK(dalloc(g, &p->chunk_row, (uint64_t)num_chunks), "cudaMalloc(chunk rows)");
   CK(dalloc(g, &p->chunk_part, (uint64_t)num_chunks), "cudaMalloc(chunk partials)");
   CK(launch_chunk_fill(p->first, nlong, p->chunk_row, g->sms, g->stream), "chunk fill");
@@ -1076,6 +1076,7 @@ int finish_create(nwgpu_graph* g, const float* weights, uint32_t flags, nwgpu_gr
   cudaError_t    e;
   int            rc;
   auto           bail = [](int code) { return code; };
+  g->finish_apart = (flags & kGraphBatchMember) != 0;
   // Merge-path sweep (graphs kept in input order, or NWGPU_SWEEP naming a
   // merge-path variant): 256-thread CTAs by default. NWGPU_SWEEP
   // (base|hot|hot512|hot1024x8), NWGPU_IPT, NWGPU_HOT_IDS, NWGPU_CTAS_PER_SM and
@@ -1150,10 +1151,6 @@ int finish_create(nwgpu_graph* g, const float* weights, uint32_t flags, nwgpu_gr
     // explicit launch settings in the environment take precedence over tuning
     const char* tune = getenv("NWGPU_AUTOTUNE");
     const bool  shapes_only = (flags & kGraphTuneShapes) && !(flags & NWGPU_GRAPH_AUTOTUNE);
-    // Graphs solved beside others on several streams: their finishing kernels run under the others' sweeps, and the
-    // tuner must not prefer the shape that holds a whole SM for being the one that can do without them (a ragged
-    // batch of 256 graphs 36.1 to 37.0 ms).
-    if (flags & kGraphTuneShapes) g->plan.bin.fused = 0u;
     const bool  want_tune = (flags & (NWGPU_GRAPH_AUTOTUNE | kGraphTuneShapes)) || (tune && !strcmp(tune, "1"));
     if (want_tune && g->bplan.ok && !getenv("NWGPU_BLOCK_LOADS") && !getenv("NWGPU_BLOCK_PIECE_ENTRIES")) {
       rc = autotune_blocked(g);  // plain solves run the blocked sweep

@@ -506,7 +506,7 @@ int nwgpu_batch_create(uint64_t num_graphs, const uint64_t* vertex_offsets, cons
   const uint32_t solo_tune = (solo_tune_env && !strcmp(solo_tune_env, "0")) ? 0u : kGraphTuneShapes;
   for (RaggedSolo& S : b->solos) {
     rc = nwgpu_graph_create(row_ptr + (vertex_offsets[S.g] + S.g), col + entry_offsets[S.g], nullptr, S.n, S.nnz,
-                            (flags & NWGPU_GRAPH_DEVICE_PTRS) | solo_tune, &S.h);
+                            (flags & NWGPU_GRAPH_DEVICE_PTRS) | kGraphBatchMember | solo_tune, &S.h);
     if (rc) {
       char msg[400];
       nwgpu_last_error(msg, sizeof(msg));

@@ -135,6 +135,7 @@ struct nwgpu_graph {
   float        tune_us = 0.f;    // the chosen parameters' time per sweep when tuned
   // Degree-binned sweep (relabelled graphs with non-increasing row lengths).
   nwgpu::BinPlan plan;
+  bool           finish_apart = false;  // kGraphBatchMember: no plan of it is fused
   // Destination-blocked sweep (plain and single-seed solves), built at creation with NWGPU_SWEEP=blocked.
   nwgpu::BlockPlan bplan;
   bool             blocked_off = false;  // this solve's degrees failed the blocked sweep's check: binned sweep
@@ -247,6 +248,12 @@ constexpr uint32_t kGraphNoBlockedPlan = 0x80000000u;
 // ranks equal an untuned handle's bit for bit (the graphs a ragged batch
 // solves alone).
 constexpr uint32_t kGraphTuneShapes = 0x40000000u;
+// Graph-creation flag for internal callers: a graph solved beside others on
+// several streams. Its sweeps keep their finishing kernels, which run under
+// the others' sweeps, and the tuner must not prefer the launch shape that holds
+// a whole SM for being the one that can do without them (a ragged batch of 256
+// graphs 36.1 to 37.0 ms).
+constexpr uint32_t kGraphBatchMember = 0x20000000u;
 // Whether a solve in `mode` over `plan` (the handle's forward plan or none) runs the blocked sweep.
 bool use_blocked(const nwgpu_graph* g, const BinPlan* plan, int mode);
 // run_sweeps' result when the degree check stopped a blocked solve before its first sweep (internal).

@@ -3,10 +3,13 @@ solve in one launch, larger ones sweep by sweep, with a finishing kernel where
 the long rows are many. The tests that compare these paths with one another
 (same ranks, bit for bit) compare nothing if a graph takes another path than
 they mean."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from nwgraph_b200 import Graph, graphs as G
+from nwgraph_b200 import _native as N
 from test_resident_gpu import KINDS, _graph
 
 pytestmark = pytest.mark.gpu
@@ -122,3 +125,22 @@ def test_finishing_work(gpu, monkeypatch, rows, per_row, kernels):
     with Graph(rp, col) as g:
         g.page_rank(deg, b, 0.85, 0.0, 7)
     assert np.array_equal(a, b)
+
+
+BATCH_MEMBER, TUNE_SHAPES = 0x20000000, 0x40000000  # nwgpu_graph_create's flags of a ragged batch's own graphs
+
+
+@pytest.mark.parametrize("flags", [BATCH_MEMBER, BATCH_MEMBER | TUNE_SHAPES, BATCH_MEMBER | N.GRAPH_AUTOTUNE])
+@pytest.mark.parametrize("tune_all", ["0", "1"])
+def test_graphs_of_a_batch_keep_the_finishing_kernel(gpu, monkeypatch, flags, tune_all):
+    """Whether they are tuned or not, and through every plan the tuner builds."""
+    monkeypatch.setenv("NWGPU_AUTOTUNE", tune_all)
+    g = G.rmat(18, 16, 4)
+    assert _kernels(g.row_ptr, g.col) <= (1 if tune_all == "0" else 2)  # a graph of its own has none in the hot shape
+    for _ in range(2):  # timed, then from the cache
+        h = C.c_void_p()
+        N.check(N.lib().nwgpu_graph_create(g.row_ptr.ctypes.data, g.col.ctypes.data, None, g.n, g.nnz, flags, C.byref(h)))
+        info = N.GraphInfo()
+        N.check(N.lib().nwgpu_graph_get_info(h, C.byref(info)))
+        N.lib().nwgpu_graph_destroy(h)
+        assert info.kernels_per_sweep == 2
