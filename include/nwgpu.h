@@ -135,7 +135,8 @@ typedef struct nwgpu_pr_stats {
   uint64_t iterations;     /* sweeps run, counting the one whose error fell below threshold */
   double   final_error;    /* L1 change of the last sweep (FP64, as page_rank.hpp:125-134) */
   int32_t  converged;      /* final_error < threshold */
-  double   device_ms;      /* CUDA-event time of the sweep loop */
+  double   device_ms;      /* time of the sweeps: CUDA events around the loop, or, where one launch runs the whole
+                              solve (kernels_per_sweep 0), the device's clock before the first and after the last */
   double   ms_per_iter;
   double   bytes_per_iter; /* algorithmic bytes of one sweep: 4 nnz + 4 (n+1) + 20 n */
   double   gteps;          /* nnz * iterations / device time */

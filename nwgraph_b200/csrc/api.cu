@@ -658,11 +658,9 @@ nwgpu_pr_options read_options(const nwgpu_pr_options* options) {
   return opt;
 }
 
-// The caller's statistics of a finished solve (ev0 to ev1), and its status.
-static int report_solve(nwgpu_graph* g, const PrState& fin, nwgpu_pr_stats* stats, cudaStream_t s) {
+// The caller's statistics of a finished solve, whose sweeps took ms, and its status.
+static int report_solve(nwgpu_graph* g, const PrState& fin, double ms, nwgpu_pr_stats* stats, cudaStream_t s) {
   if (stats) {
-    float ms = 0.f;
-    cudaEventElapsedTime(&ms, g->ev0, g->ev1);
     stats->iterations = fin.iter;
     stats->final_error = fin.last_error;
     stats->converged = (int32_t)fin.converged;
@@ -724,7 +722,11 @@ static int solve_resident(nwgpu_graph* g, const uint32_t* out_degree, float* ran
   if (!device_ptrs)
     CK(cudaMemcpyAsync(g->stage_u32, out_degree, n * sizeof(uint32_t), cudaMemcpyHostToDevice, s), "copy out_degree");
   *g->h_st = PrState{};
-  CK(cudaEventRecord(g->ev0, s), "cudaEventRecord");
+  // the sweeps' time: the launch also reads the degrees and writes the ranks, which the loop's events leave out
+  static_assert(sizeof(PrState) + sizeof(unsigned long long) <= kHostBlock, "the state and the time beside it");
+  volatile unsigned long long* const ns = reinterpret_cast<unsigned long long*>(g->h_st + 1);
+  a.sweeps_ns = reinterpret_cast<unsigned long long*>(g->d_hst + 1);
+  double ms = 0.0;
   do {
     a.turn = p.turn;
     a.chunk_end = a.iter0 + kGraphChunk;
@@ -737,14 +739,14 @@ static int solve_resident(nwgpu_graph* g, const uint32_t* out_degree, float* ran
     CK(e, "pr_resident");
     *ran = true;
     p.turn ^= 1u;
-    CK(cudaEventRecord(g->ev1, s), "cudaEventRecord");
     if (!device_ptrs) CK(cudaMemcpyAsync(ranks, a.out, n * sizeof(float), cudaMemcpyDeviceToHost, s), "copy ranks");
     CK(cudaStreamSynchronize(s), "pr_resident");
+    if (g->h_st->iter > a.iter0) ms += 1e-6 * (double)*ns;
     a.iter0 = g->h_st->iter;
   } while (!g->h_st->done);
   const PrState fin = *g->h_st;
   if (fin.fault) return fail(NWGPU_ERR_CUDA, "a bounded device wait gave up (fault word %u)", fin.fault);
-  return report_solve(g, fin, stats, s);
+  return report_solve(g, fin, ms, stats, s);
 }
 
 // Shared body of nwgpu_pr_run (uniform teleport) and nwgpu_ppr_run (one-hot).
@@ -841,7 +843,9 @@ int solve_single(nwgpu_graph* g, const uint32_t* out_degree, float* ranks, float
   }
   CK(cudaStreamSynchronize(s), "copy ranks");
   trace.mark("ranks out");
-  return report_solve(g, fin, stats, s);
+  float ms = 0.f;
+  cudaEventElapsedTime(&ms, g->ev0, g->ev1);
+  return report_solve(g, fin, (double)ms, stats, s);
 }
 
 }  // namespace nwgpu

@@ -47,6 +47,12 @@ __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
   return v;
 }
 
+__device__ __forceinline__ unsigned long long clock_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
+}
+
 // Place of the CTA's entry e in s_val: one spare word per 32, so that lanes
 // reading every fourth entry hit 32 banks.
 __device__ __forceinline__ uint32_t skew(uint32_t e) { return e + (e >> 5); }
@@ -129,6 +135,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) pr_resident_kernel(const 
   __shared__ uint32_t      s_seed, s_bins;
   __shared__ uint32_t      s_bin[kNumBins][3];  // the bins the CTA has rows of: bin, first row, end
   __shared__ int           s_done, s_fault;
+  __shared__ unsigned long long s_start;
   const int                tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const uint32_t           cta = blockIdx.x, ctas = gridDim.x;
   const uint32_t           ra = a.bounds[cta], rb = a.bounds[cta + 1], R = rb - ra;
@@ -193,6 +200,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) pr_resident_kernel(const 
     return s_fault == 0;
   };
   bool ok = barrier();
+  if (cta == 0 && tid == 0) s_start = clock_ns();
 
   unsigned long long it = a.iter0;
   while (ok) {
@@ -217,6 +225,7 @@ __global__ void __launch_bounds__(kResidentThreads, 1) pr_resident_kernel(const 
             a.state->converged = conv ? 1u : 0u;
             a.state->aborted = (abort_seen && !conv) ? 1u : 0u;
             a.state->done = s_done ? 1u : 0u;
+            *a.sweeps_ns = clock_ns() - s_start;
           }
         }
       }

@@ -34,6 +34,7 @@ struct ResidentArgs {
   unsigned int    turn;
   double*         part;
   PrState*        state;     // host-mapped: written once, at the end
+  unsigned long long* sweeps_ns;  // beside it: from the first sweep's start to the last one's residual
   double*         err_hist;
   uint32_t        err_cap;
   const volatile unsigned int* abort_word;

@@ -144,3 +144,20 @@ def test_graphs_of_a_batch_keep_the_finishing_kernel(gpu, monkeypatch, flags, tu
         N.check(N.lib().nwgpu_graph_get_info(h, C.byref(info)))
         N.lib().nwgpu_graph_destroy(h)
         assert info.kernels_per_sweep == 2
+
+
+def test_device_ms_is_the_sweeps(gpu):
+    """Also where one launch reads the degrees, sweeps and writes the ranks: 1 sweep takes what each of 40 takes (the
+    launch's start and end take about 20 us, a sweep 14), and no sweep takes no time."""
+    g = G.grid(1_000_000)
+    deg = g.out_degree()
+    out = np.empty(g.n, np.float32)
+    with Graph(g.row_ptr, g.col) as h:
+        per = {its: min(h.page_rank(deg, out, 0.85, -1.0, its).ms_per_iter for _ in range(9)) for its in (1, 40)}
+        assert h.info()["kernels_per_sweep"] == 0
+        none = h.page_rank(deg, out, 0.85, -1.0, 0)
+        long = h.page_rank(deg, out, 0.85, -1.0, 4100)  # two launches
+    print(per, long.ms_per_iter)
+    assert 0.5 * per[40] < per[1] < 1.5 * per[40]
+    assert 0.5 * per[40] < long.ms_per_iter < 1.5 * per[40]
+    assert none.device_ms == 0.0 and none.ms_per_iter == 0.0
