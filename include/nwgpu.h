@@ -314,6 +314,13 @@ int nwgpu_abort(nwgpu_graph* g);
  * long that took. Nothing faults; the context stays usable. */
 int nwgpu_selftest_bounded_wait(uint32_t polls, uint32_t* gave_up, double* ms);
 
+/* Self-test of the grid barriers of a small graph's one-launch solve. They give
+ * up after 2^22 polls. This runs such a solve (g: kernels_per_sweep 0 after a
+ * solve of its own; host arrays as for nwgpu_pr_run) whose barriers wait for
+ * one more CTA than there is, with `polls` polls (1 .. 2^20): it must end with
+ * NWGPU_ERR_CUDA, what it leaves in ranks is undefined, and g solves on. */
+int nwgpu_selftest_resident_wait(nwgpu_graph* g, const uint32_t* out_degree, float* ranks, uint32_t polls);
+
 /* Self-test of the engine's behaviour when memory runs out: of the calling
  * thread's allocations of device memory or of small pinned host blocks, the
  * one after `after` more fails, once, as if the memory were not there (the

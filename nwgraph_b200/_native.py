@@ -116,6 +116,7 @@ SIGNATURES = {
                                        C.c_uint64, _vp, C.POINTER(PrStats)]),
     "nwgpu_abort": (C.c_int, [_vp]),
     "nwgpu_selftest_bounded_wait": (C.c_int, [C.c_uint32, C.POINTER(C.c_uint32), C.POINTER(C.c_double)]),
+    "nwgpu_selftest_resident_wait": (C.c_int, [_vp, _vp, _vp, C.c_uint32]),
     "nwgpu_selftest_fail_allocation": (C.c_int, [C.c_int64]),
     "nwgpu_spmv": (C.c_int, [_vp, _vp, _vp, C.POINTER(PrOptions)]),
     "nwgpu_release_cached_memory": (C.c_int, []),

@@ -683,9 +683,11 @@ static int report_solve(nwgpu_graph* g, const PrState& fin, double ms, nwgpu_pr_
 // A plain or single-seed solve as resident launches (one, unless it takes more
 // than kGraphChunk sweeps). *ran stays false, with nothing done, where the
 // device cannot hold the grid at once; the caller then runs the sweep loop.
+// missing CTAs (the self-test's) make every grid barrier give up after `polls`.
 static int solve_resident(nwgpu_graph* g, const uint32_t* out_degree, float* ranks, float damping, float threshold,
                           uint64_t max_iters, bool device_ptrs, int teleport, uint32_t seed, float init, float base,
-                          cudaStream_t s, nwgpu_pr_stats* stats, bool* ran) {
+                          cudaStream_t s, nwgpu_pr_stats* stats, bool* ran, unsigned missing = 0,
+                          unsigned polls = kBarrierPolls) {
   ResidentPlan&     p = g->resident;
   const BinnedArgs& b = g->plan.bin;
   const uint64_t    n = g->n;
@@ -700,6 +702,8 @@ static int solve_resident(nwgpu_graph* g, const uint32_t* out_degree, float* ran
   a.contrib1 = g->contrib[1];
   a.bounds = p.bounds;
   a.sync = p.sync;
+  a.arrivals = (unsigned)p.ctas + missing;
+  a.polls = polls;
   a.part = p.part;
   a.state = g->d_hst;
   a.err_hist = g->err_hist;
@@ -938,6 +942,17 @@ int nwgpu_selftest_bounded_wait(uint32_t polls, uint32_t* gave_up, double* ms) {
   *gave_up = flag;
   *ms = t;
   return NWGPU_OK;
+}
+
+int nwgpu_selftest_resident_wait(nwgpu_graph* g, const uint32_t* out_degree, float* ranks, uint32_t polls) {
+  clear_error();
+  if (!g || !out_degree || !ranks) return fail(NWGPU_ERR_INVALID_ARG, "NULL argument");
+  if (polls == 0 || polls > (1u << 20)) return fail(NWGPU_ERR_INVALID_ARG, "polls = %u outside [1, 2^20]", polls);
+  if (!g->resident.ok)
+    return fail(NWGPU_ERR_INVALID_ARG, "no solve of this graph has run in one launch (kernels_per_sweep 0)");
+  bool ran = false;
+  return solve_resident(g, out_degree, ranks, 0.85f, 0.f, 1, false, kTeleportUniform, 0u, (float)(1.0 / (double)g->n), 0.f,
+                        g->stream, nullptr, &ran, 1u, polls);
 }
 
 int nwgpu_selftest_fail_allocation(int64_t after) {

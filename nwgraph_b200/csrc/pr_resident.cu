@@ -39,7 +39,6 @@ constexpr uint32_t kWarps = kResidentThreads / 32;
 constexpr int      kIdRegs = 8;               // column ids a thread keeps
 constexpr uint32_t kRowCost = 3;              // a row's update, in entries
 constexpr uint32_t kItemsPerCta = 2048;       // at least this much work per CTA
-constexpr unsigned kBarrierPolls = 1u << 22;  // about 3 s: then the solve ends with an error
 
 __device__ __forceinline__ unsigned int ld_acquire(const unsigned int* p) {
   unsigned int v;
@@ -185,13 +184,13 @@ __global__ void __launch_bounds__(kResidentThreads, 1) pr_resident_kernel(const 
   // All CTAs' writes before it are seen by all CTAs after it. False once a wait gave up.
   auto barrier = [&]() {
     __syncthreads();
-    target += ctas;
-    if (tid == 0 && ctas > 1u) {
+    target += a.arrivals;
+    if (tid == 0 && a.arrivals > 1u) {
       __threadfence();
       atomicAdd(a.sync + a.turn, 1u);
       unsigned polls = 0;
       while (ld_acquire(a.sync + a.turn) < target)
-        if (++polls == kBarrierPolls) {
+        if (++polls == a.polls) {
           s_fault = 1;
           break;
         }
