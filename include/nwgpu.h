@@ -117,7 +117,15 @@ int nwgpu_graph_get_info(const nwgpu_graph* g, nwgpu_graph_info* info);
 
 /* Solve modes */
 #define NWGPU_MODE_PARITY 0u     /* page_rank_v10 semantics: Jacobi, leak (no dangling redistribution) */
-/* Launch strategies */
+/* Launch strategies. NWGPU_LAUNCH_GRAPH: a handle's first loop launches its
+ * sweeps itself (a one-shot call then builds no graph), the second builds the
+ * loop's graph, which takes about 0.2 ms once. A small graph's plain and
+ * single-seed solves (kernels_per_sweep 0) are one cooperative launch each over
+ * up to all SMs: it starts when every CTA of it finds room beside what else
+ * runs and holds that room to its end, so such solves on several handles take
+ * turns solve by solve, not sweep by sweep, and one waits for any kernel that
+ * fills an SM. A caller whose own kernel does that until a solve returns must
+ * solve with NWGPU_LAUNCH_STREAM. */
 #define NWGPU_LAUNCH_GRAPH 0u    /* CUDA graph; device-side while loop, convergence tested on the GPU */
 #define NWGPU_LAUNCH_STREAM 1u   /* one kernel per sweep on the stream; sweeps after convergence exit at once */
 

@@ -683,11 +683,9 @@ static int report_solve(nwgpu_graph* g, const PrState& fin, double ms, nwgpu_pr_
 // A plain or single-seed solve as resident launches (one, unless it takes more
 // than kGraphChunk sweeps). *ran stays false, with nothing done, where the
 // device cannot hold the grid at once; the caller then runs the sweep loop.
-// missing CTAs (the self-test's) make every grid barrier give up after `polls`.
 static int solve_resident(nwgpu_graph* g, const uint32_t* out_degree, float* ranks, float damping, float threshold,
                           uint64_t max_iters, bool device_ptrs, int teleport, uint32_t seed, float init, float base,
-                          cudaStream_t s, nwgpu_pr_stats* stats, bool* ran, unsigned missing = 0,
-                          unsigned polls = kBarrierPolls) {
+                          cudaStream_t s, nwgpu_pr_stats* stats, bool* ran, unsigned selftest_polls = 0) {
   ResidentPlan&     p = g->resident;
   const BinnedArgs& b = g->plan.bin;
   const uint64_t    n = g->n;
@@ -702,8 +700,7 @@ static int solve_resident(nwgpu_graph* g, const uint32_t* out_degree, float* ran
   a.contrib1 = g->contrib[1];
   a.bounds = p.bounds;
   a.sync = p.sync;
-  a.arrivals = (unsigned)p.ctas + missing;
-  a.polls = polls;
+  a.polls = selftest_polls;
   a.part = p.part;
   a.state = g->d_hst;
   a.err_hist = g->err_hist;
@@ -952,7 +949,7 @@ int nwgpu_selftest_resident_wait(nwgpu_graph* g, const uint32_t* out_degree, flo
     return fail(NWGPU_ERR_INVALID_ARG, "no solve of this graph has run in one launch (kernels_per_sweep 0)");
   bool ran = false;
   return solve_resident(g, out_degree, ranks, 0.85f, 0.f, 1, false, kTeleportUniform, 0u, (float)(1.0 / (double)g->n), 0.f,
-                        g->stream, nullptr, &ran, 1u, polls);
+                        g->stream, nullptr, &ran, polls);
 }
 
 int nwgpu_selftest_fail_allocation(int64_t after) {

@@ -32,8 +32,7 @@ struct ResidentArgs {
   const uint32_t* bounds;
   unsigned int*   sync;
   unsigned int    turn;
-  unsigned int    arrivals;  // CTAs a grid barrier waits for (all of them; one more in the self-test)
-  unsigned int    polls;     // a barrier's polls before the solve ends with an error
+  unsigned int    polls;     // the self-test's, whose barriers wait for one CTA too many and give up after so many; else 0
   double*         part;
   PrState*        state;     // host-mapped: written once, at the end
   unsigned long long* sweeps_ns;  // beside it: from the first sweep's start to the last one's residual
@@ -55,7 +54,7 @@ struct ResidentArgs {
   uint32_t        hub_ids;
 };
 
-constexpr unsigned int kBarrierPolls = 1u << 22;  // about 3 s
+constexpr unsigned int kBarrierPolls = 1u << 22;  // about 3 s: then the solve ends with an error
 constexpr unsigned int kFaultResidentWait = 0x52455349u;  // PrState::fault: a grid barrier gave up
 
 // Largest entry count the resident solve is considered for.
