@@ -155,6 +155,7 @@ int build_gmres(nwgpu_graph* g) {
     CK(host_block_get((void**)&b.h_dots[i]), "cudaHostAlloc(gmres dots)");
     CK(cudaHostGetDevicePointer((void**)&b.d_hdots[i], b.h_dots[i], 0), "cudaHostGetDevicePointer(gmres dots)");
   }
+  CK(cudaStreamSynchronize(g->stream), "gmres buffers");  // cleared before the caller's stream writes them
   b.gmres_ready = true;
   return NWGPU_OK;
 }
@@ -364,7 +365,10 @@ extern "C" int nwgpu_pr_vjp(nwgpu_graph* g, const float* ranks, const float* dL_
   }
   // gradients from the adjoint l (in g->rank)
   if (dL_dw) {
-    if (!opt.device_ptrs && !b.gw) CK(dalloc(g, &b.gw, nnz), "cudaMalloc(dL/dw staging)");
+    if (!opt.device_ptrs && !b.gw) {
+      CK(dalloc(g, &b.gw, nnz), "cudaMalloc(dL/dw staging)");
+      CK(cudaStreamSynchronize(g->stream), "dL/dw staging");  // cleared before the caller's stream writes it
+    }
     float* dst = opt.device_ptrs ? dL_dw : b.gw;
     CK(launch_vjp_grad_w(b.t, g->g.col, g->g.emap, b.r_int, g->rank, b.vbase, n, nnz, damping, b.f, b.q, dst, g->sms, s),
        "dL/dw");
