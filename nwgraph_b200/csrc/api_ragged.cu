@@ -244,7 +244,7 @@ int build_union(RaggedBatch* b, const std::vector<uint32_t>& ids, const std::vec
   cudaError_t    e = launch_union_build(b->graphs, b->row_ptr, b->col, p, rp, col, sms, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   int rc = e == cudaSuccess ? nwgpu_graph_create(rp, col, nullptr, n, nnz,
-                                                 NWGPU_GRAPH_DEVICE_PTRS | kGraphNoBlockedPlan | tune, &U->h)
+                                                 NWGPU_GRAPH_DEVICE_PTRS | kGraphNoBlockedPlan | kGraphBatchMember | tune, &U->h)
                             : cuda_fail(e, "union CSR");
   pool_free(rp, s);
   pool_free(col, s);

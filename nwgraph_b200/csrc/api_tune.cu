@@ -45,6 +45,14 @@ struct Choice {
   uint32_t long_row = kLongRow, chunk = kChunk, bin0_rows = kBin0Rows;
 };
 
+// A batch member's candidates of the hot shape count as this much slower than
+// they measured by themselves: beside others, CTAs that hold a whole SM cost
+// more. It decides the unions too, whose sweeps always run in that shape but
+// stage nothing with the other one's tiers. The two shapes time alike there
+// (175.7 to 177.1 us a sweep, 2^23 vertices) and the choice was a coin's toss: a
+// ragged batch of 256 graphs 35.7 ms one way, 36.4 the other.
+constexpr float kHotBeside = 1.05f;
+
 std::mutex                    g_mu;
 std::map<std::string, Choice> g_cache;
 bool                          g_loaded = false;
@@ -350,12 +358,13 @@ int autotune_binned(nwgpu_graph* g, bool shapes_only) {
     c.bin0_rows = bin0_rows;
     cands.push_back(c);
   }
+  const auto cost = [&](const Choice& c) { return c.us * (g->finish_apart && c.hot ? kHotBeside : 1.f); };
   for (Choice c : cands) {
     if ((rc = apply(g, c))) return rc;
     float us = 0.f;
     if ((rc = time_plan(g, a, sweeps, &us))) return rc;
     c.us = us;
-    if (us < best.us) best = c;
+    if (cost(c) < cost(best)) best = c;
   }
   if ((rc = apply(g, best))) return rc;
   g->tuned = 1;
