@@ -409,7 +409,7 @@ void ResidentPlan::release(cudaStream_t s) {
   *this = ResidentPlan();
 }
 
-// The resident solve's plan, once per graph: relabelled graphs on the binned
+// The resident solve's plan: relabelled graphs on the binned
 // sweep (not one that NWGPU_SWEEP names) of which every CTA's rows and entries
 // fit its shared memory. The hubs staged beside them are those that save the
 // most: a sweep's gathers past them cost about a clock each per SM, staging
@@ -429,10 +429,8 @@ void ResidentPlan::release(cudaStream_t s) {
 // gathers on, where no room is left for hubs (none lies between) -- unless one
 // CTA has most of the work: 0.73 with 34,000 entries beside an average of
 // 2300, 0.92 with 30,000 beside 8300, but 1.19 beside 15,000.
-static int ensure_resident(nwgpu_graph* g) {
+static int plan_resident(nwgpu_graph* g) {
   ResidentPlan& p = g->resident;
-  if (p.tried) return NWGPU_OK;
-  p.tried = true;
   if (!g->relabelled || !g->plan.ok || g->bplan.ok || g->n == 0 || g->nnz > kResidentMaxEntries ||
       g->n > kResidentMaxEntries || getenv("NWGPU_SWEEP"))
     return NWGPU_OK;
@@ -483,6 +481,25 @@ static int ensure_resident(nwgpu_graph* g) {
   p.ctas = C;
   p.ok = true;
   return NWGPU_OK;
+}
+
+// Without a plan nothing of it is kept, and the sweep loop solves the graph:
+// also where there was no memory for one.
+static int ensure_resident(nwgpu_graph* g) {
+  ResidentPlan& p = g->resident;
+  if (p.tried) return NWGPU_OK;
+  const uint64_t held = g->device_bytes;
+  int            rc = plan_resident(g);
+  if (!p.ok) {
+    p.release(g->stream);
+    g->device_bytes = held;
+  }
+  p.tried = true;
+  if (rc == NWGPU_ERR_OUT_OF_MEMORY) {
+    clear_error();
+    rc = NWGPU_OK;
+  }
+  return rc;
 }
 
 // Sweep grid of a binned solve: the plan's, except the weighted and adjoint

@@ -59,7 +59,7 @@ constexpr unsigned int kFaultResidentWait = 0x52455349u;  // PrState::fault: a g
 
 // Largest entry count the resident solve is considered for.
 constexpr uint64_t kResidentMaxEntries = 8ull << 20;
-// What the fullest CTA may gather past the hubs per sweep (ensure_resident has the measurements): of any graph, in
+// What the fullest CTA may gather past the hubs per sweep (plan_resident has the measurements): of any graph, in
 // sectors; of one with long rows and no CTA above kResidentUneven times the average, in gathers.
 constexpr uint32_t kResidentSectors = 17000;
 constexpr uint32_t kResidentSkewedGathers = 33000;

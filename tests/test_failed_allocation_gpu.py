@@ -92,3 +92,22 @@ def test_the_call_after_a_failed_one(gpu, call, relabel):
     finally:
         N.lib().nwgpu_selftest_fail_allocation(-1)
     assert 10 <= failed < 200
+
+
+def test_no_memory_for_the_small_graph_plan(gpu):
+    """The plan of the one-launch solve is an extra: without memory for it the first solve runs the sweep loop."""
+    out, want = np.empty(RMAT.n, np.float32), np.empty(RMAT.n, np.float32)
+    solve_buffers = 12  # ensure_solve_buffers' allocations, before the plan's four
+    try:
+        for after in range(solve_buffers, solve_buffers + 5):
+            with Graph(RMAT.row_ptr, RMAT.col) as g, Graph(RMAT.row_ptr, RMAT.col) as loop:
+                loop.page_rank(DEG, want, 0.85, 1e-6, 50, launch="stream")
+                N.lib().nwgpu_selftest_fail_allocation(after)
+                g.page_rank(DEG, out, 0.85, 1e-6, 50)
+                N.lib().nwgpu_selftest_fail_allocation(-1)
+                without = after < solve_buffers + 4
+                assert g.info()["kernels_per_sweep"] == (1 if without else 0)
+                assert not without or g.info()["device_bytes"] == loop.info()["device_bytes"]
+                assert np.array_equal(out, want)
+    finally:
+        N.lib().nwgpu_selftest_fail_allocation(-1)
